@@ -29,9 +29,10 @@ struct yv_renderer {
   yv_light light;
   LaunchCfg cfg;
   // device scene
-  uint32_t* d_words = nullptr;
-  uint32_t* d_orig = nullptr;
-  uint4* d_attrs = nullptr;  // shading records, 16 B per leaf
+  uint2* d_nodes = nullptr;  // node records, 8 B each
+  uint2* d_cold = nullptr;   // their cold records, 8 B each
+  uint32_t* d_leaf_attr = nullptr;  // leaf -> attribute, or null
+  uint4* d_attrs = nullptr;  // shading records, 16 B per attribute
   uint32_t* d_node_data = nullptr;  // level-of-detail attribute per node, or null
   size_t cap_nodes = 0, cap_attrs = 0;  // allocated records of the three
   float detail = 0.f;  // SVORenderer::m_detailCoef; 0 = exact leaves
@@ -42,6 +43,7 @@ struct yv_renderer {
   SvoDeviceScene scene;
   bool has_scene = false;
   uint64_t scene_bytes = 0;
+  uint32_t scene_nodes = 0;  // nodes of the scene (shared ones once)
   // renderer-owned frame buffer (RendererBase::m_colorBuf) and scratch
   uint32_t* d_rgba = nullptr;
   size_t rgba_cap = 0;
@@ -67,18 +69,21 @@ static yv_status cuda_fail(cudaError_t e, const char* what) {
   } while (0)
 
 static void free_scene(yv_renderer* r) {
-  cudaFree(r->d_words);
-  cudaFree(r->d_orig);
+  cudaFree(r->d_nodes);
+  cudaFree(r->d_cold);
+  cudaFree(r->d_leaf_attr);
   cudaFree(r->d_attrs);
   cudaFree(r->d_node_data);
-  r->d_words = nullptr;
-  r->d_orig = nullptr;
+  r->d_nodes = nullptr;
+  r->d_cold = nullptr;
+  r->d_leaf_attr = nullptr;
   r->d_attrs = nullptr;
   r->d_node_data = nullptr;
   r->cap_nodes = r->cap_attrs = 0;
   r->has_scene = false;
   r->scene = SvoDeviceScene();
   r->scene_bytes = 0;
+  r->scene_nodes = 0;
   r->dyn = nullptr;
 }
 
@@ -91,7 +96,7 @@ static SvoDeviceScene scene_of(const yv_renderer* r) {
   uint32_t count = 0, root = YV_EMPTY_NODE, nattrs = 0;
   yv_svo_dynamic_device(r->dyn, &nodes, &count, &root, &attrs, &nattrs);
   SvoDeviceScene sc;
-  sc.nodes = reinterpret_cast<const uint4*>(nodes);
+  sc.nodes = nodes;
   sc.attrs = attrs;
   sc.n_nodes = count;
   sc.n_attrs = nattrs;
@@ -104,10 +109,10 @@ namespace yv {
 
 // Scene buffers for a scene built on the device: waits for the renderer's
 // last frame, drops the current scene and returns buffers for nn node
-// records (8 child words + id each) and na shading records, reusing the
+// records (and their cold records) and na shading records, reusing the
 // existing allocations when they are large enough.
-yv_status renderer_scene_buffers(yv_renderer* r, uint32_t nn, uint32_t na, uint32_t** words,
-                                 uint32_t** orig, void** attrs) {
+yv_status renderer_scene_buffers(yv_renderer* r, uint32_t nn, uint32_t na, uint2** nodes,
+                                 uint2** cold, void** attrs) {
   YV_CUDA(cudaSetDevice(r->device), "cudaSetDevice");
   if (r->frame_pending) cudaStreamSynchronize(r->last_stream);
   r->has_scene = false;
@@ -115,14 +120,16 @@ yv_status renderer_scene_buffers(yv_renderer* r, uint32_t nn, uint32_t na, uint3
   r->dyn = nullptr;
   cudaFree(r->d_node_data);
   r->d_node_data = nullptr;
+  cudaFree(r->d_leaf_attr);
+  r->d_leaf_attr = nullptr;
   const size_t want_n = nn ? nn : 1, want_a = na ? na : 1;
   if (want_n > r->cap_nodes) {
-    cudaFree(r->d_words);
-    cudaFree(r->d_orig);
-    r->d_words = r->d_orig = nullptr;
+    cudaFree(r->d_nodes);
+    cudaFree(r->d_cold);
+    r->d_nodes = r->d_cold = nullptr;
     r->cap_nodes = 0;
-    YV_CUDA(cudaMalloc(&r->d_words, want_n * 32u), "cudaMalloc(nodes)");
-    YV_CUDA(cudaMalloc(&r->d_orig, want_n * 4u), "cudaMalloc(ids)");
+    YV_CUDA(cudaMalloc(&r->d_nodes, want_n * 8u), "cudaMalloc(nodes)");
+    YV_CUDA(cudaMalloc(&r->d_cold, want_n * 8u), "cudaMalloc(ids)");
     r->cap_nodes = want_n;
   }
   if (want_a > r->cap_attrs) {
@@ -132,21 +139,22 @@ yv_status renderer_scene_buffers(yv_renderer* r, uint32_t nn, uint32_t na, uint3
     YV_CUDA(cudaMalloc(&r->d_attrs, want_a * 16u), "cudaMalloc(attrs)");
     r->cap_attrs = want_a;
   }
-  *words = r->d_words;
-  *orig = r->d_orig;
+  *nodes = r->d_nodes;
+  *cold = r->d_cold;
   *attrs = r->d_attrs;
   return YV_OK;
 }
 
 // Makes the buffers filled after renderer_scene_buffers the current scene.
 void renderer_commit_scene(yv_renderer* r, uint32_t nn, uint32_t na, uint32_t root_word) {
-  r->scene.nodes = reinterpret_cast<const uint4*>(r->d_words);
-  r->scene.orig_id = r->d_orig;
+  r->scene.nodes = r->d_nodes;
+  r->scene.cold = r->d_cold;
   r->scene.attrs = r->d_attrs;
   r->scene.n_nodes = nn;
   r->scene.n_attrs = na;
   r->scene.root_word = root_word;
-  r->scene_bytes = (uint64_t)nn * 36u + (uint64_t)na * 16u;
+  r->scene_bytes = (uint64_t)nn * 16u + (uint64_t)na * 16u;
+  r->scene_nodes = nn;
   r->has_scene = true;
 }
 
@@ -225,11 +233,11 @@ static yv_status set_scene_impl(yv_renderer* r, const yv_vox_node* nodes, uint32
   }
   std::vector<uint32_t> node_data;
   if (lod) {
-    node_data.resize(dl.orig_id.size());
+    node_data.resize(dl.records());
     for (size_t i = 0; i < node_data.size(); ++i) {
-      node_data[i] = nodes[dl.orig_id[i]].data;
+      node_data[i] = nodes[dl.cold[2 * i]].data;
       if (node_data[i] >= nattrs) {
-        set_last_error("level-of-detail attribute of node " + std::to_string(dl.orig_id[i]) +
+        set_last_error("level-of-detail attribute of node " + std::to_string(dl.cold[2 * i]) +
                        " out of range");
         return YV_ERR_BAD_POOL;
       }
@@ -238,14 +246,19 @@ static yv_status set_scene_impl(yv_renderer* r, const yv_vox_node* nodes, uint32
   YV_CUDA(cudaSetDevice(r->device), "cudaSetDevice");
   if (r->frame_pending) cudaStreamSynchronize(r->last_stream);
   free_scene(r);
-  const size_t nn = dl.orig_id.size();
+  const size_t nn = dl.records(), nl = dl.leaf_attr.size();
   if (nn) {
-    YV_CUDA(cudaMalloc(&r->d_words, nn * 32u), "cudaMalloc(nodes)");
-    YV_CUDA(cudaMalloc(&r->d_orig, nn * 4u), "cudaMalloc(orig)");
-    YV_CUDA(cudaMemcpy(r->d_words, dl.words.data(), nn * 32u, cudaMemcpyHostToDevice),
+    YV_CUDA(cudaMalloc(&r->d_nodes, nn * 8u), "cudaMalloc(nodes)");
+    YV_CUDA(cudaMalloc(&r->d_cold, nn * 8u), "cudaMalloc(ids)");
+    YV_CUDA(cudaMemcpy(r->d_nodes, dl.nodes.data(), nn * 8u, cudaMemcpyHostToDevice),
             "upload nodes");
-    YV_CUDA(cudaMemcpy(r->d_orig, dl.orig_id.data(), nn * 4u, cudaMemcpyHostToDevice),
+    YV_CUDA(cudaMemcpy(r->d_cold, dl.cold.data(), nn * 8u, cudaMemcpyHostToDevice),
             "upload ids");
+  }
+  if (nl) {
+    YV_CUDA(cudaMalloc(&r->d_leaf_attr, nl * 4u), "cudaMalloc(leaves)");
+    YV_CUDA(cudaMemcpy(r->d_leaf_attr, dl.leaf_attr.data(), nl * 4u, cudaMemcpyHostToDevice),
+            "upload leaves");
   }
   if (nattrs) {
     // Per leaf: RGBA8 + the unit normal, normalised here once with the
@@ -273,13 +286,15 @@ static yv_status set_scene_impl(yv_renderer* r, const yv_vox_node* nodes, uint32
   }
   r->cap_nodes = nn;
   r->cap_attrs = nattrs;
-  r->scene.nodes = reinterpret_cast<const uint4*>(r->d_words);
-  r->scene.orig_id = r->d_orig;
+  r->scene.nodes = r->d_nodes;
+  r->scene.cold = r->d_cold;
+  r->scene.leaf_attr = r->d_leaf_attr;
   r->scene.attrs = r->d_attrs;
   r->scene.n_nodes = (uint32_t)nn;
   r->scene.n_attrs = nattrs;
   r->scene.root_word = dl.root_word;
-  r->scene_bytes = (uint64_t)nn * 36u + (uint64_t)nattrs * 16u;
+  r->scene_bytes = (uint64_t)nn * 16u + (uint64_t)nl * 4u + (uint64_t)nattrs * 16u;
+  r->scene_nodes = dl.n_unique;
   if (lod && nn) {
     YV_CUDA(cudaMalloc(&r->d_node_data, nn * 4u), "cudaMalloc(node data)");
     YV_CUDA(cudaMemcpy(r->d_node_data, node_data.data(), nn * 4u, cudaMemcpyHostToDevice),
@@ -440,7 +455,7 @@ yv_status yv_get_ray_basis(const yv_renderer* r, float dir0[3], float du[3], flo
 
 yv_status yv_get_device_scene_info(const yv_renderer* r, uint64_t* nodes, uint64_t* bytes) {
   if (!r || !nodes || !bytes) return YV_ERR_INVALID_ARG;
-  *nodes = scene_of(r).n_nodes;
+  *nodes = r->dyn ? scene_of(r).n_nodes : r->scene_nodes;
   *bytes = r->scene_bytes;
   return YV_OK;
 }

@@ -53,9 +53,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) batch_kernel(BatchLaunch b) {
   int item = 0;
   Trace tr;
   float dx = 0.f, dy = 0.f, dz = 0.f;
-  uint32_t hitw = 0xFFFFFFFFu, fp = 0;
-  float ht = 0.f;
-  uint4 attr = make_uint4(0u, 0u, 0u, 0u);
+  uint32_t lit = 0, dark = 0;
 
   for (;;) {
     const uint32_t busy = __ballot_sync(0xFFFFFFFFu, mode == kPrimary || mode == kShadow);
@@ -64,10 +62,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) batch_kernel(BatchLaunch b) {
       // so keeps it out of the registers while a brick tile is marched.
       tr = Trace{};
       dx = dy = dz = 0.f;
-      hitw = 0xFFFFFFFFu;
-      fp = 0;
-      ht = 0.f;
-      attr = make_uint4(0u, 0u, 0u, 0u);
+      lit = dark = 0;
       // the whole warp takes the next 8x4 tile of the queue
       uint32_t base = 0;
       if (lane == 0) base = atomicAdd(&b.counters[0], 32u);
@@ -84,11 +79,11 @@ __global__ void __launch_bounds__(256, kMinBlocks) batch_kernel(BatchLaunch b) {
         off = (uint32_t)y * (uint32_t)it.width + (uint32_t)x;
         if (it.kind == kBatchSvo) {
           pixel_dir(it.fa, x, y, dx, dy, dz);
-          if (begin_trace(it.svo, it.fa.pos[0], it.fa.pos[1], it.fa.pos[2], dx, dy, dz, tr,
+          if (begin_trace(it.svo, nullptr, 0u, it.fa.pos[0], it.fa.pos[1], it.fa.pos[2], dx, dy, dz, tr,
                           err)) {
             mode = kPrimary;
           } else {
-            write_pixel(it.fa, off, 0u, 0xFFFFFFFFu, 0.f, tr.fetches, 0u);
+            write_miss(it.fa, off, tr.fetches);
           }
         } else {
           float o[3], d[3];
@@ -119,40 +114,33 @@ __global__ void __launch_bounds__(256, kMinBlocks) batch_kernel(BatchLaunch b) {
                                           leaf, err);
     if (r == kContinue) continue;
     if (mode == kShadow) {
-      write_pixel(it.fa, off, shade(attr, it.fa, r == kHit), hitw, ht, fp, tr.fetches, attr);
+      write_color(it.fa, off, r == kHit ? dark : lit, tr.fetches);
       mode = kIdle;
     } else if (r == kMiss) {
-      write_pixel(it.fa, off, 0u, 0xFFFFFFFFu, 0.f, tr.fetches, 0u);
+      write_miss(it.fa, off, tr.fetches);
       mode = kIdle;
     } else {
-      hitw = (__ldg(it.svo.orig_id + tr.node) << 3) | (tr.ch ^ tr.df);
-      ht = max3f(tr.t.x1, tr.t.y1, tr.t.z1);
-      fp = tr.fetches;
-      attr = make_uint4(0u, 0u, 0u, 0u);
+      const uint32_t hitw = hit_word<false>(it.svo, tr, leaf);
+      const float ht = max3f(tr.t.x1, tr.t.y1, tr.t.z1);
+      uint4 attr = make_uint4(0u, 0u, 0u, 0u);
       if (leaf < it.svo.n_attrs)
         attr = load_shading<false>(it.svo, leaf);
       else
         err |= YV_DEV_ERR_POOL;
+      write_primary(it.fa, off, hitw, ht, tr.fetches, attr);
+      lit = shade(attr, it.fa, false);
       mode = kIdle;
       if (!it.fa.shadows) {
-        write_pixel(it.fa, off, shade(attr, it.fa, false), hitw, ht, fp, 0u, attr);
+        write_color(it.fa, off, lit, 0u);
       } else {
+        dark = shade(attr, it.fa, true);
         float o[3];
-        o[0] = __fadd_rn(it.fa.pos[0], __fmul_rn(dx, ht));
-        o[1] = __fadd_rn(it.fa.pos[1], __fmul_rn(dy, ht));
-        o[2] = __fadd_rn(it.fa.pos[2], __fmul_rn(dz, ht));
-        int e = 0;
-        float m = tr.t.x1;
-        if (tr.t.y1 > m) { e = 1; m = tr.t.y1; }
-        if (tr.t.z1 > m) e = 2;
-        const float half = __int_as_float((127 - (tr.level + 2)) << 23);
-        const float d_off = ((tr.df >> e) & 1u) ? half : -half;
-        o[e] = __fadd_rn(o[e], d_off);
-        if (begin_trace(it.svo, o[0], o[1], o[2], it.fa.light_ray[0], it.fa.light_ray[1],
-                        it.fa.light_ray[2], tr, err))
+        shadow_origin(it.fa, tr, dx, dy, dz, ht, o);
+        if (begin_trace(it.svo, nullptr, 0u, o[0], o[1], o[2], it.fa.light_ray[0],
+                        it.fa.light_ray[1], it.fa.light_ray[2], tr, err))
           mode = kShadow;
         else
-          write_pixel(it.fa, off, shade(attr, it.fa, false), hitw, ht, fp, tr.fetches, attr);
+          write_color(it.fa, off, lit, tr.fetches);
       }
     }
   }

@@ -418,21 +418,29 @@ __global__ void emit_leaves_kernel(Grid g, const uint64_t* list, uint32_t m,
   }
 }
 
-// Renderer layout: 32-byte child-word records, identity id map, 16-byte
-// shading records (RGBA8 + unit normal, the FP32 normalisation of the
-// upload path).
-__global__ void device_layout_kernel(const yv_vox_node* nodes, uint32_t nn, uint32_t* words,
-                                     uint32_t* orig) {
+// Renderer layout: 8-byte node records and their cold records (node and
+// leaf children are already numbered consecutively), 16-byte shading records
+// (RGBA8 + unit normal, the FP32 normalisation of the upload path).
+__global__ void device_layout_kernel(const yv_vox_node* nodes, uint32_t nn, uint2* rec,
+                                     uint2* cold) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
     const yv_vox_node v = nodes[i];
+    uint32_t codes = 0, rank = 0, first = 0, leaf = 0, leaves = 0;
 #pragma unroll
     for (int ch = 0; ch < 8; ++ch) {
       const uint32_t w = v.child[ch];
-      words[8 * (size_t)i + ch] = ((v.flags >> ch) & 1u) ? (YV_DW_LEAF | w)
-                                  : (w & 0x80000000u)     ? YV_DW_NULL
-                                                          : w;
+      uint32_t k = YV_CODE_NULL;
+      if ((v.flags >> ch) & 1u) {
+        k = YV_CODE_LEAF;
+        if (!leaves++) leaf = w;
+      } else if (!(w & 0x80000000u)) {
+        if (!rank) first = w;
+        k = rank++;
+      }
+      codes |= k << (28 - 4 * ch);
     }
-    orig[i] = i;
+    rec[i] = make_uint2(first, codes);
+    cold[i] = make_uint2(i, leaf);
   }
 }
 
@@ -624,14 +632,14 @@ yv_status yv_set_scene_dense(yv_renderer* r, const float* density, const uint8_t
   yv_status st = build_dense(density, rgb, depth, iso, s, res);
   if (st != YV_OK) return st;
   // renderer layout, written into the renderer's (reused) scene buffers
-  uint32_t *words = nullptr, *orig = nullptr;
+  uint2 *nodes = nullptr, *cold = nullptr;
   void* rec = nullptr;
-  st = renderer_scene_buffers(r, res.nn, res.na, &words, &orig, &rec);
+  st = renderer_scene_buffers(r, res.nn, res.na, &nodes, &cold, &rec);
   if (st != YV_OK) return st;
   cudaError_t e = cudaSuccess;
   if (res.nn) {
     device_layout_kernel<<<grid_for(res.nn), 256, 0, s>>>(res.nodes.as<yv_vox_node>(), res.nn,
-                                                          words, orig);
+                                                          nodes, cold);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess && res.na) {

@@ -935,8 +935,10 @@ namespace yv {
 yv_status build_device_layout(const yv_vox_node* nodes, uint32_t count,
                               uint32_t root, uint32_t nattrs,
                               DeviceLayout* out, std::string* why) {
-  out->words.clear();
-  out->orig_id.clear();
+  out->nodes.clear();
+  out->cold.clear();
+  out->leaf_attr.clear();
+  out->n_unique = 0;
   out->root_word = YV_DW_NULL;
   out->depth = 0;
   if (root & 0x80000000u) return YV_OK;  // null root: empty scene
@@ -998,40 +1000,54 @@ yv_status build_device_layout(const yv_vox_node* nodes, uint32_t count,
     st.pop_back();
   }
   out->depth = height[root];
-  // breadth-first numbering of the reachable nodes
-  std::vector<uint32_t> newid(count, 0xFFFFFFFFu);
-  std::vector<uint32_t> order;
+  // breadth-first records: the run of a node's children is laid down when its
+  // first record is reached (run[id]), and shared by its other records
+  std::vector<uint32_t> run(count, 0xFFFFFFFFu), leaves(count, 0);
+  std::vector<uint32_t> order;  // record -> caller node id
   order.push_back(root);
-  newid[root] = 0;
+  uint64_t n_leaves = 0;
   for (size_t i = 0; i < order.size(); ++i) {
-    const yv_vox_node& n = nodes[order[i]];
+    const uint32_t id = order[i];
+    if (run[id] != 0xFFFFFFFFu) continue;
+    const yv_vox_node& n = nodes[id];
+    run[id] = (uint32_t)order.size();
+    leaves[id] = (uint32_t)n_leaves;
+    ++out->n_unique;
     for (int ch = 0; ch < 8; ++ch) {
-      uint32_t w = n.child[ch];
-      if (((n.flags >> ch) & 1u) || (w & 0x80000000u)) continue;
-      if (newid[w] == 0xFFFFFFFFu) {
-        newid[w] = (uint32_t)order.size();
+      const uint32_t w = n.child[ch];
+      if ((n.flags >> ch) & 1u) {
+        out->leaf_attr.push_back(w);
+        ++n_leaves;
+      } else if (!(w & 0x80000000u)) {
         order.push_back(w);
       }
     }
-  }
-  if (order.size() > YV_MAX_DEVICE_NODES) {
-    *why = "pool larger than 2^29 nodes";
-    return YV_ERR_BAD_POOL;
-  }
-  out->words.resize(order.size() * 8);
-  out->orig_id = order;
-  for (size_t i = 0; i < order.size(); ++i) {
-    const yv_vox_node& n = nodes[order[i]];
-    for (int ch = 0; ch < 8; ++ch) {
-      uint32_t w = n.child[ch], dw;
-      if ((n.flags >> ch) & 1u)
-        dw = YV_DW_LEAF | w;
-      else if (w & 0x80000000u)
-        dw = YV_DW_NULL;
-      else
-        dw = newid[w];
-      out->words[i * 8 + (size_t)ch] = dw;
+    if (order.size() > YV_MAX_DEVICE_NODES || n_leaves > 0xFFFFFFFEull) {
+      *why = "pool larger than 2^29 nodes";
+      return YV_ERR_BAD_POOL;
     }
+  }
+  bool same = true;  // leaves already numbered as their attributes
+  for (size_t i = 0; i < out->leaf_attr.size() && same; ++i) same = out->leaf_attr[i] == i;
+  if (same) out->leaf_attr.clear();
+  out->nodes.resize(order.size() * 2);
+  out->cold.resize(order.size() * 2);
+  for (size_t i = 0; i < order.size(); ++i) {
+    const uint32_t id = order[i];
+    const yv_vox_node& n = nodes[id];
+    uint32_t codes = 0, rank = 0;
+    for (int ch = 0; ch < 8; ++ch) {
+      uint32_t k = YV_CODE_NULL;
+      if ((n.flags >> ch) & 1u)
+        k = YV_CODE_LEAF;
+      else if (!(n.child[ch] & 0x80000000u))
+        k = rank++;
+      codes |= k << (28 - 4 * ch);
+    }
+    out->nodes[2 * i] = run[id];
+    out->nodes[2 * i + 1] = codes;
+    out->cold[2 * i] = id;
+    out->cold[2 * i + 1] = leaves[id];
   }
   out->root_word = 0;
   return YV_OK;

@@ -59,7 +59,7 @@ template <int kMinBlocks, bool kStaged, bool kLod = false, bool kRef = false>
 static cudaError_t launch_with(const SvoDeviceScene& sc, const SvoFrameArgs& a, int bt,
                                uint32_t nsm, uint32_t refill, int per_sm, cudaStream_t stream) {
   auto kern = svo_frame_kernel<kMinBlocks, kRef, kSvoRing, kStaged, kLod>;
-  const size_t smem = (size_t)nsm * 32u + (size_t)(bt / 32) * kSvoRing * 1024u;
+  const size_t smem = (size_t)(nsm / 2) * 16u + (size_t)(bt / 32) * kSvoRing * 1024u;
   if (smem > 48u * 1024u) {
     static bool opted_in[64] = {false};
     int dev = 0;

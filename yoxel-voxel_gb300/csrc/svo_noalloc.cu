@@ -83,8 +83,7 @@ extern "C" yv_status yv_render_svo_noalloc(const yv_vox_node* nodes, uint32_t co
   if (st != YV_OK) return st;
 
   SvoDeviceScene sc;
-  sc.nodes = reinterpret_cast<const uint4*>(nodes);  // read as 40-byte VoxNode records
-  sc.orig_id = nullptr;
+  sc.nodes = nodes;  // read as 40-byte VoxNode records
   sc.attrs = attrs;
   sc.n_nodes = count;
   sc.n_attrs = nattrs;

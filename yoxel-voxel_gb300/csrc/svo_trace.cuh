@@ -15,12 +15,18 @@
 //    the slowest ray of a tile and the shadow rays of some lanes overlap the
 //    primary rays of others.  Consecutive ray ids map to 8x4 pixel tiles, so
 //    lanes refilled together trace neighbouring pixels;
-//  * node records are 32 B (one L2 sector); a traversal step reads the one
-//    32-bit child word it tests (the sector stays in L1 while the ray is in
-//    the node).  Staging the breadth-first first `smem_nodes` records (the
-//    top tree levels) in shared memory is a separately compiled variant the
-//    launch configuration can ask for; reading every record through L1
-//    measured as fast or faster, so it is off by default;
+//  * node records are 8 B, four to an L2 sector: the record of the first
+//    child and a nibble per child that tells node, leaf and null apart.  A
+//    ray reads a record when it enters (or returns to) a node and keeps it in
+//    two registers, so a step over a null child reads no memory.  Against
+//    32-byte records of 8 child words read at every step (2048^3 terrain,
+//    1920x1080, shadow rays): with the updates below 598 -> 524 us, a
+//    160x120 frame 71 -> 60 us; bit masks and a popcount in place of the
+//    nibbles cost more than the loads saved (575 us).
+//    Staging the breadth-first first `smem_nodes` records (the top tree
+//    levels) in shared memory is a separately compiled variant the launch
+//    configuration can ask for; reading every record through L1 measured as
+//    fast or faster, so it is off by default;
 //  * the recursion of RecTrace becomes an explicit per-lane stack of
 //    (node id, child, slab box) frames, so a pop restores the parent's exact
 //    float values: every operation is an explicit round-to-nearest intrinsic
@@ -43,7 +49,9 @@ namespace yv {
 namespace {
 
 constexpr uint32_t kFetchCap = 1u << 20;
-// traversal steps between two warp votes (refill / end-of-ray handling)
+// traversal steps between two warp votes (refill / end-of-ray handling); 12
+// measured slower (576 against 524 us on a 1920x1080 frame with shadow rays).
+// Unrolled 4 deep: 8 copies of the step overflow the instruction cache.
 constexpr int kStepsPerVote = 8;
 
 struct Box {
@@ -57,65 +65,70 @@ __device__ __forceinline__ float max3f(float a, float b, float c) {
 // Minimum / maximum for the comparisons of the traversal (slab values are
 // never NaN; +0 and -0 compare equal, so the choice between them is moot).
 __device__ __forceinline__ float fmin3(float a, float b, float c) {
-  return fminf(fminf(a, b), c);
+  float m;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+  return m;
 }
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
-  return fmaxf(fmaxf(a, b), c);
+  float m;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+  return m;
 }
 
-// FindFirstChild (cell/spu/trace_spu.cpp:48-68).
+// FindFirstChild (cell/spu/trace_spu.cpp:48-68).  The traversal is bound by
+// the half-rate ALU pipe (compares, selects, logic), so the box updates here
+// and in `advance` are written as predicated moves and FP32 adds, which the
+// compiler's selects would put on that pipe.
 __device__ __forceinline__ uint32_t ffc(Box& t) {
   const float te = fmax3(t.x1, t.y1, t.z1);
-  uint32_t ch = 0;
-  float tm = __fmul_rn(0.5f, __fadd_rn(t.x1, t.x2));
-  if (te > tm) { ch |= 1u; t.x1 = tm; } else { t.x2 = tm; }
-  tm = __fmul_rn(0.5f, __fadd_rn(t.y1, t.y2));
-  if (te > tm) { ch |= 2u; t.y1 = tm; } else { t.y2 = tm; }
-  tm = __fmul_rn(0.5f, __fadd_rn(t.z1, t.z2));
-  if (te > tm) { ch |= 4u; t.z1 = tm; } else { t.z2 = tm; }
+  uint32_t ch;
+  asm("{\n\t.reg .pred px, py, pz;\n\t.reg .f32 mx, my, mz;\n\t"
+      "add.rn.f32 mx, %1, %4;\n\tadd.rn.f32 my, %2, %5;\n\tadd.rn.f32 mz, %3, %6;\n\t"
+      "mul.rn.f32 mx, mx, 0f3F000000;\n\tmul.rn.f32 my, my, 0f3F000000;\n\t"
+      "mul.rn.f32 mz, mz, 0f3F000000;\n\t"
+      "setp.gt.f32 px, %7, mx;\n\tsetp.gt.f32 py, %7, my;\n\tsetp.gt.f32 pz, %7, mz;\n\t"
+      "@px mov.f32 %1, mx;\n\t@!px mov.f32 %4, mx;\n\t"
+      "@py mov.f32 %2, my;\n\t@!py mov.f32 %5, my;\n\t"
+      "@pz mov.f32 %3, mz;\n\t@!pz mov.f32 %6, mz;\n\t"
+      "selp.u32 %0, 4, 0, px;\n\t@py or.b32 %0, %0, 8;\n\t@pz or.b32 %0, %0, 16;\n\t}"
+      : "=&r"(ch), "+f"(t.x1), "+f"(t.y1), "+f"(t.z1), "+f"(t.x2), "+f"(t.y2), "+f"(t.z2)
+      : "f"(te));
   return ch;
 }
 
 // GoNext (cell/spu/trace_spu.cpp:70-93) in two parts: the exit axis (the
-// argmin tie order of :75-78) and the move into the sibling across it.
-__device__ __forceinline__ int exit_axis(const Box& t) {
-  if (t.x2 > t.y2) return (t.y2 < t.z2) ? 1 : 2;
-  return (t.x2 < t.z2) ? 0 : 2;
+// argmin tie order of :75-78) as the child bit it flips, and the move into
+// the sibling across it.
+__device__ __forceinline__ uint32_t exit_bit(const Box& t) {
+  const bool p = t.x2 > t.y2;
+  const bool ey = p && t.y2 < t.z2;
+  const bool ex = !p && t.x2 < t.z2;
+  return ey ? 8u : (ex ? 4u : 16u);
 }
 
-__device__ __forceinline__ void advance(uint32_t& ch, Box& t, int e) {
-  // branch-free: the lanes of a warp cross different axes
-  ch ^= 1u << e;
-  const bool ex = e == 0, ey = e == 1, ez = e == 2;
-  const float a1 = ex ? t.x1 : (ey ? t.y1 : t.z1);
-  const float a2 = ex ? t.x2 : (ey ? t.y2 : t.z2);
-  const float n2 = __fadd_rn(a2, __fsub_rn(a2, a1));
-  t.x1 = ex ? a2 : t.x1;
-  t.x2 = ex ? n2 : t.x2;
-  t.y1 = ey ? a2 : t.y1;
-  t.y2 = ey ? n2 : t.y2;
-  t.z1 = ez ? a2 : t.z1;
-  t.z2 = ez ? n2 : t.z2;
+// On the crossed axis t1, t2 <- t2, t2 + (t2 - t1); predicated, the lanes of
+// a warp cross different axes.
+__device__ __forceinline__ void advance(uint32_t& ch, Box& t, uint32_t bit) {
+  ch ^= bit;
+  asm("{\n\t.reg .pred px, py, pz;\n\t.reg .f32 dx, dy, dz;\n\t"
+      "setp.eq.u32 px, %6, 4;\n\tsetp.eq.u32 py, %6, 8;\n\tsetp.eq.u32 pz, %6, 16;\n\t"
+      "sub.rn.f32 dx, %3, %0;\n\tsub.rn.f32 dy, %4, %1;\n\tsub.rn.f32 dz, %5, %2;\n\t"
+      "@px mov.f32 %0, %3;\n\t@py mov.f32 %1, %4;\n\t@pz mov.f32 %2, %5;\n\t"
+      "@px add.rn.f32 %3, %3, dx;\n\t@py add.rn.f32 %4, %4, dy;\n\t"
+      "@pz add.rn.f32 %5, %5, dz;\n\t}"
+      : "+f"(t.x1), "+f"(t.y1), "+f"(t.z1), "+f"(t.x2), "+f"(t.y2), "+f"(t.z2)
+      : "r"(bit));
 }
 
-// Child word c of node id, read where it lies at every step (the node's
-// sector stays in L1 while the ray is inside it, so the 8 words are not
-// held in registers).  kRef = false: the library's 32-byte device records
-// (top levels from shared memory).  kRef = true: the reference's 40-byte
-// VoxNode {flags, data, child[8]} read in place, its leaf / null flags
-// folded into the same word encoding.
-// kStaged: the first nsm records are read from shared memory.
-template <bool kRef, bool kStaged>
-__device__ __forceinline__ uint32_t child_word(const SvoDeviceScene& sc, const uint32_t* sm,
-                                               uint32_t nsm, uint32_t id, uint32_t c) {
-  if (kRef) {
-    const uint32_t* p = reinterpret_cast<const uint32_t*>(sc.nodes) + 10 * (size_t)id;
-    const uint32_t fl = __ldg(p);
-    const uint32_t cw = __ldg(p + 2 + c);
-    return ((fl >> c) & 1u) ? (YV_DW_LEAF | cw) : ((cw & 0x80000000u) ? YV_DW_NULL : cw);
-  }
-  if (kStaged && id < nsm) return sm[8 * id + c];
-  return __ldg(reinterpret_cast<const uint32_t*>(sc.nodes) + 8 * (size_t)id + c);
+// Child word c of node id of a caller's pool, whose flags word is fl: the
+// reference's 40-byte VoxNode {flags, data, child[8]} read in place, its leaf
+// and null children folded into one encoding (a child is null by its word,
+// whatever the flags say).
+__device__ __forceinline__ uint32_t ref_child_word(const SvoDeviceScene& sc, uint32_t id,
+                                                   uint32_t fl, uint32_t c) {
+  const uint32_t cw =
+      __ldg(reinterpret_cast<const uint32_t*>(sc.nodes) + 10 * (size_t)id + 2 + c);
+  return ((fl >> c) & 1u) ? (YV_DW_LEAF | cw) : ((cw & 0x80000000u) ? YV_DW_NULL : cw);
 }
 
 // Nanoseconds of the GPU's global timer.
@@ -131,18 +144,25 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
 // Levels whose current child is the last one the ray crosses are never
 // pushed: returning to them would only return further.
 struct __align__(16) Frame {
-  uint32_t idch;  // node << 3 | ch
+  uint32_t node;
   float x1, y1, z1;
   float x2, y2, z2;
-  uint32_t level;
+  uint32_t chlev;  // child (x 4) | level << 8
 };
 
 enum : uint32_t { kIdle = 0, kPrimary = 1, kShadow = 2, kDone = 3 };
 enum : int { kContinue = 0, kHit = 1, kMiss = 2 };
+// trace_step's `leaf` for a leaf child of the library's layout: its attribute
+// is looked up once, at the end of the ray (hit_leaf)
+constexpr uint32_t kLeafOfNode = 0xFFFFFFFFu;
 
 // Traversal state of one lane.
 struct Trace {
+  // current child and direction mirror, both x 4: bits 2, 3 and 4 for x, y, z
   uint32_t node, ch, df, fetches;
+  // the node's record (first node child, child codes); a caller's VoxNode:
+  // its flags
+  uint32_t first, codes;
   uint32_t sp;  // frames held
   uint32_t lo;  // with a shared-memory ring: frames below lo are in local memory
   int level;
@@ -164,17 +184,17 @@ __device__ __forceinline__ void push_frame(Frame* stk, uint4* ring, Trace& tr, c
     const uint32_t s = tr.lo & (uint32_t)(kRing - 1);
     const uint4 q0 = ring[(2 * s) * 32], q1 = ring[(2 * s + 1) * 32];
     Frame g;
-    g.idch = q0.x;
+    g.node = q0.x;
     g.x1 = __uint_as_float(q0.y); g.y1 = __uint_as_float(q0.z); g.z1 = __uint_as_float(q0.w);
     g.x2 = __uint_as_float(q1.x); g.y2 = __uint_as_float(q1.y); g.z2 = __uint_as_float(q1.z);
-    g.level = q1.w;
+    g.chlev = q1.w;
     stk[tr.lo++] = g;
   }
   const uint32_t s = tr.sp & (uint32_t)(kRing - 1);
   ring[(2 * s) * 32] =
-      make_uint4(f.idch, __float_as_uint(f.x1), __float_as_uint(f.y1), __float_as_uint(f.z1));
+      make_uint4(f.node, __float_as_uint(f.x1), __float_as_uint(f.y1), __float_as_uint(f.z1));
   ring[(2 * s + 1) * 32] =
-      make_uint4(__float_as_uint(f.x2), __float_as_uint(f.y2), __float_as_uint(f.z2), f.level);
+      make_uint4(__float_as_uint(f.x2), __float_as_uint(f.y2), __float_as_uint(f.z2), f.chlev);
   ++tr.sp;
 }
 
@@ -189,23 +209,41 @@ __device__ __forceinline__ Frame pop_frame(const Frame* stk, const uint4* ring, 
   const uint32_t s = tr.sp & (uint32_t)(kRing - 1);
   const uint4 q0 = ring[(2 * s) * 32], q1 = ring[(2 * s + 1) * 32];
   Frame g;
-  g.idch = q0.x;
+  g.node = q0.x;
   g.x1 = __uint_as_float(q0.y); g.y1 = __uint_as_float(q0.z); g.z1 = __uint_as_float(q0.w);
   g.x2 = __uint_as_float(q1.x); g.y2 = __uint_as_float(q1.y); g.z2 = __uint_as_float(q1.z);
-  g.level = q1.w;
+  g.chlev = q1.w;
   return g;
 }
 
 
+// Reads what the traversal keeps of the node tr.node.
+// kStaged: the first nsm records are read from shared memory.
+template <bool kRef, bool kStaged>
+__device__ __forceinline__ void enter_node(const SvoDeviceScene& sc, const uint32_t* sm,
+                                           uint32_t nsm, Trace& tr) {
+  if (kRef) {
+    tr.codes = __ldg(reinterpret_cast<const uint32_t*>(sc.nodes) + 10 * (size_t)tr.node);
+    return;
+  }
+  const uint2 v = (kStaged && tr.node < nsm)
+                      ? reinterpret_cast<const uint2*>(sm)[tr.node]
+                      : __ldg(reinterpret_cast<const uint2*>(sc.nodes) + tr.node);
+  tr.first = v.x;
+  tr.codes = v.y;
+}
+
 // SetupTrace (reaction/report/voxel.tex:312-326) + RecTrace entry test
 // (cell/ppu_renderer.cpp:20-21) + the root fetch.  False: the ray misses.
-__device__ __forceinline__ bool begin_trace(const SvoDeviceScene& sc, float px, float py, float pz,
+template <bool kRef = false, bool kStaged = false>
+__device__ __forceinline__ bool begin_trace(const SvoDeviceScene& sc, const uint32_t* sm,
+                                            uint32_t nsm, float px, float py, float pz,
                                             float dx, float dy, float dz, Trace& tr,
                                             uint32_t& err) {
   uint32_t df = 0;
-  if (dx < 0.f) { px = __fsub_rn(1.f, px); dx = -dx; df |= 1u; }
-  if (dy < 0.f) { py = __fsub_rn(1.f, py); dy = -dy; df |= 2u; }
-  if (dz < 0.f) { pz = __fsub_rn(1.f, pz); dz = -dz; df |= 4u; }
+  if (dx < 0.f) { px = __fsub_rn(1.f, px); dx = -dx; df |= 4u; }
+  if (dy < 0.f) { py = __fsub_rn(1.f, py); dy = -dy; df |= 8u; }
+  if (dz < 0.f) { pz = __fsub_rn(1.f, pz); dz = -dz; df |= 16u; }
   Box R;
   R.x1 = __fdiv_rn(__fsub_rn(0.f, px), dx);
   R.x2 = __fdiv_rn(__fsub_rn(1.f, px), dx);
@@ -227,9 +265,38 @@ __device__ __forceinline__ bool begin_trace(const SvoDeviceScene& sc, float px, 
   tr.sp = 0;
   tr.lo = 0;
   tr.fetches = 1;
+  enter_node<kRef, kStaged>(sc, sm, nsm, tr);
   tr.t = R;
   tr.ch = ffc(tr.t);
   return true;
+}
+
+// What the ray may do at its current child: the child ahead of the ray's
+// origin (or, for a primary ray, a leaf behind it) is a hit or a descent, any
+// other is passed over.
+struct Probe {
+  bool leaf;   // a leaf child (else a node where `take` is set)
+  bool take;   // the ray hits it or descends into it
+  uint32_t w;  // the node child's code in the top nibble; caller's pool: the
+               // child word
+};
+
+template <bool kRef>
+__device__ __forceinline__ Probe probe_child(const SvoDeviceScene& sc, const Trace& tr,
+                                             bool cull) {
+  Probe p;
+  const uint32_t c = tr.ch ^ tr.df;
+  const bool ahead = fmin3(tr.t.x2, tr.t.y2, tr.t.z2) > 0.f;
+  if (kRef) {
+    p.w = ref_child_word(sc, tr.node, tr.codes, c >> 2);
+    p.leaf = (p.w & YV_DW_LEAF) != 0u;
+    p.take = p.leaf ? (!cull || ahead) : (!(p.w & YV_DW_NULL) && ahead);
+  } else {
+    p.w = tr.codes << c;
+    p.leaf = p.w >= (YV_CODE_LEAF << 28);
+    p.take = p.leaf ? (!cull || ahead) : ((int32_t)p.w >= 0 && ahead);
+  }
+  return p;
 }
 
 // One step of RecTrace: test the current child (leaf -> hit, subtree ->
@@ -250,18 +317,17 @@ __device__ __forceinline__ int trace_step(const SvoDeviceScene& sc, const uint32
                                           uint32_t nsm, Frame* stk, uint4* ring, Trace& tr,
                                           bool cull, uint32_t& leaf, uint32_t& err,
                                           float lod_coef = 0.f) {
-  const uint32_t w = child_word<kRef, kStaged>(sc, sm, nsm, tr.node, tr.ch ^ tr.df);
-  const bool ahead = fmin3(tr.t.x2, tr.t.y2, tr.t.z2) > 0.f;
+  const Probe p = probe_child<kRef>(sc, tr, cull);
   // exit axis of the current child and whether it is the last one along
   // the ray in this node (needed by both the descent and the sibling move)
-  int e = exit_axis(tr.t);
-  const bool last = (tr.ch >> e) & 1u;
-  if (w & YV_DW_LEAF) {
-    if (!cull || ahead) {
-      leaf = w & 0x7FFFFFFFu;
+  uint32_t e = exit_bit(tr.t);
+  const bool last = (tr.ch & e) != 0u;
+  if (p.take) {
+    if (p.leaf) {
+      leaf = kRef ? (p.w & 0x7FFFFFFFu) : kLeafOfNode;
       return kHit;
     }
-  } else if (!(w & YV_DW_NULL) && ahead) {
+    const uint32_t w = kRef ? p.w : tr.first + (p.w >> 28);
     if (kLod) {
       const float side = __int_as_float((126 - tr.level) << 23);  // 2^-(level+1)
       const float te = fmaxf(fmax3(tr.t.x1, tr.t.y1, tr.t.z1), 0.f);
@@ -288,26 +354,28 @@ __device__ __forceinline__ int trace_step(const SvoDeviceScene& sc, const uint32
     ++tr.fetches;
     if (!last) {
       Frame f;
-      f.idch = (tr.node << 3) | tr.ch;
+      f.node = tr.node;
       f.x1 = tr.t.x1; f.y1 = tr.t.y1; f.z1 = tr.t.z1;
       f.x2 = tr.t.x2; f.y2 = tr.t.y2; f.z2 = tr.t.z2;
-      f.level = (uint32_t)tr.level;
+      f.chlev = tr.ch | ((uint32_t)tr.level << 8);
       push_frame<kRing>(stk, ring, tr, f);
     }
     ++tr.level;
     tr.node = w;
+    enter_node<kRef, kStaged>(sc, sm, nsm, tr);
     tr.ch = ffc(tr.t);
     return kContinue;
   }
   if (last) {
     if (tr.sp == 0) return kMiss;
     const Frame f = pop_frame<kRing>(stk, ring, tr);
-    tr.ch = f.idch & 7u;
-    tr.node = f.idch >> 3;
-    tr.level = (int)f.level;
+    tr.node = f.node;
+    enter_node<kRef, kStaged>(sc, sm, nsm, tr);
+    tr.ch = f.chlev & 0xFFu;
+    tr.level = (int)(f.chlev >> 8);
     tr.t.x1 = f.x1; tr.t.y1 = f.y1; tr.t.z1 = f.z1;
     tr.t.x2 = f.x2; tr.t.y2 = f.y2; tr.t.z2 = f.z2;
-    e = exit_axis(tr.t);
+    e = exit_bit(tr.t);
   }
   advance(tr.ch, tr.t, e);
   return kContinue;
@@ -357,6 +425,23 @@ __device__ __forceinline__ uint4 load_shading(const SvoDeviceScene& sc, uint32_t
   return __ldg(static_cast<const uint4*>(sc.attrs) + leaf);
 }
 
+// Hit word of a ray that ended at child tr.ch of tr.node, and its attribute:
+// `leaf` as trace_step left it.
+template <bool kRef>
+__device__ __forceinline__ uint32_t hit_word(const SvoDeviceScene& sc, const Trace& tr,
+                                             uint32_t& leaf) {
+  const uint32_t c = tr.ch ^ tr.df;  // x 4
+  if (kRef) return (tr.node << 3) | (c >> 2);
+  const uint2 cold = __ldg(sc.cold + tr.node);
+  if (leaf == kLeafOfNode) {
+    // leaf codes (both top bits of the nibble) of the children before this one
+    const uint32_t before = tr.codes & (tr.codes << 1) & 0x88888888u & ~(0xFFFFFFFFu >> c);
+    leaf = cold.y + __popc(before);
+    if (sc.leaf_attr) leaf = __ldg(sc.leaf_attr + leaf);
+  }
+  return (cold.x << 3) | (c >> 2);
+}
+
 // Lambert: ambient + diffuse*max(0, n.L) (ambient only in shadow).
 __device__ __forceinline__ uint32_t shade(uint4 at, const SvoFrameArgs& a, bool shadowed) {
   const float ndl = __fadd_rn(__fadd_rn(__fmul_rn(__uint_as_float(at.y), a.light[0]),
@@ -374,22 +459,50 @@ __device__ __forceinline__ uint32_t shade(uint4 at, const SvoFrameArgs& a, bool 
   return out;
 }
 
-// `at` is the hit leaf's shading record (zero for a miss): its normal goes to
-// the optional per-pixel normal output.
-__device__ __forceinline__ void write_pixel(const SvoFrameArgs& a, uint32_t off, uint32_t rgba,
-                                            uint32_t hitw, float ht, uint32_t f, uint32_t fs,
-                                            uint4 at = make_uint4(0u, 0u, 0u, 0u)) {
-  if (a.rgba) a.rgba[off] = rgba;
+// What a pixel's primary ray gives: hit word, t, fetches and the normal of
+// the hit leaf's shading record `at` (zero for a miss).
+__device__ __forceinline__ void write_primary(const SvoFrameArgs& a, uint32_t off,
+                                              uint32_t hitw, float ht, uint32_t f,
+                                              uint4 at = make_uint4(0u, 0u, 0u, 0u)) {
   if (a.hit) a.hit[off] = hitw;
   if (a.hit_t) a.hit_t[off] = ht;
   if (a.fetches) a.fetches[off] = f;
-  if (a.shadow_fetches) a.shadow_fetches[off] = fs;
   if (a.normal) {
     const size_t n = 3u * (size_t)off;  // off < 2^31: 3 off needs 64 bits
     a.normal[n] = __uint_as_float(at.y);
     a.normal[n + 1u] = __uint_as_float(at.z);
     a.normal[n + 2u] = __uint_as_float(at.w);
   }
+}
+
+// What is known once its shadow ray has ended too (or there is none).
+__device__ __forceinline__ void write_color(const SvoFrameArgs& a, uint32_t off, uint32_t rgba,
+                                            uint32_t fs) {
+  if (a.rgba) a.rgba[off] = rgba;
+  if (a.shadow_fetches) a.shadow_fetches[off] = fs;
+}
+
+__device__ __forceinline__ void write_miss(const SvoFrameArgs& a, uint32_t off, uint32_t f) {
+  write_primary(a, off, 0xFFFFFFFFu, 0.f, f);
+  write_color(a, off, 0u, 0u);
+}
+
+// Origin of the shadow ray of the hit tr ended at: the hit point of the
+// primary ray (pos + d t) moved half a leaf out through the entry face.
+__device__ __forceinline__ void shadow_origin(const SvoFrameArgs& a, const Trace& tr, float dx,
+                                              float dy, float dz, float ht, float* o) {
+  o[0] = __fadd_rn(a.pos[0], __fmul_rn(dx, ht));
+  o[1] = __fadd_rn(a.pos[1], __fmul_rn(dy, ht));
+  o[2] = __fadd_rn(a.pos[2], __fmul_rn(dz, ht));
+  int e = 0;
+  float m = tr.t.x1;
+  if (tr.t.y1 > m) { e = 1; m = tr.t.y1; }
+  if (tr.t.z1 > m) e = 2;
+  const float half = __int_as_float((127 - (tr.level + 2)) << 23);
+  const float d_off = ((tr.df >> (2 + e)) & 1u) ? half : -half;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if (e == i) o[i] = __fadd_rn(o[i], d_off);
 }
 
 // kMinBlocks: resident 256-thread blocks per SM the register allocation is
@@ -400,7 +513,7 @@ __device__ __forceinline__ void write_pixel(const SvoFrameArgs& a, uint32_t off,
 // kStaged: the first nsm node records are copied to shared memory and read
 // there (measured: reading every record through L1 is as fast or faster,
 // so the default is unstaged and nsm = 0).
-// Dynamic shared memory = 32 B x nsm staged nodes + 1 KB x kRing per warp.
+// Dynamic shared memory = 8 B x nsm staged nodes + 1 KB x kRing per warp.
 // kLod: level-of-detail cut-off (a.lod_coef, sc.node_data; library layout).
 template <int kMinBlocks, bool kRef, int kRing, bool kStaged, bool kLod = false>
 __global__ void __launch_bounds__(256, kMinBlocks)
@@ -410,12 +523,14 @@ __global__ void __launch_bounds__(256, kMinBlocks)
   // in a register of the traversal)
   __shared__ unsigned long long deadline;
   if (!kStaged) nsm = 0;
-  for (uint32_t i = threadIdx.x; i < 2 * nsm; i += blockDim.x) smem[i] = __ldg(sc.nodes + i);
+  nsm &= ~1u;  // whole 16-byte pairs of records
+  for (uint32_t i = threadIdx.x; i < nsm / 2; i += blockDim.x)
+    smem[i] = __ldg(reinterpret_cast<const uint4*>(sc.nodes) + i);
   if (threadIdx.x == 0 && a.budget_us)
     deadline = global_timer_ns() + 1000ull * (unsigned long long)a.budget_us;
   __syncthreads();
   const uint32_t* smw = reinterpret_cast<const uint32_t*>(smem);
-  uint4* ring = smem + 2 * nsm + (threadIdx.x >> 5) * (2 * kRing * 32) + (threadIdx.x & 31u);
+  uint4* ring = smem + nsm / 2 + (threadIdx.x >> 5) * (2 * kRing * 32) + (threadIdx.x & 31u);
 
   Frame stk[YV_MAX_DEPTH];
   const uint32_t lane = threadIdx.x & 31u;
@@ -427,9 +542,8 @@ __global__ void __launch_bounds__(256, kMinBlocks)
   uint32_t mode = kIdle, off = 0;
   Trace tr;
   float dx = 0.f, dy = 0.f, dz = 0.f;
-  uint32_t hitw = 0xFFFFFFFFu, fp = 0;
-  float ht = 0.f;
-  uint4 attr = make_uint4(0u, 0u, 0u, 0u);
+  // colours of the pixel whose shadow ray is under way, lit and in shadow
+  uint32_t lit = 0, dark = 0;
 
   for (;;) {
     // ---- refill idle lanes from the global ray counter ----
@@ -456,10 +570,11 @@ __global__ void __launch_bounds__(256, kMinBlocks)
           if (x < a.width && y < a.height) {
             off = (uint32_t)y * (uint32_t)a.width + (uint32_t)x;
             pixel_dir(a, x, y, dx, dy, dz);
-            if (begin_trace(sc, a.pos[0], a.pos[1], a.pos[2], dx, dy, dz, tr, err)) {
+            if (begin_trace<kRef, kStaged>(sc, smw, nsm, a.pos[0], a.pos[1], a.pos[2], dx, dy,
+                                           dz, tr, err)) {
               mode = kPrimary;
             } else {
-              write_pixel(a, off, 0u, 0xFFFFFFFFu, 0.f, tr.fetches, 0u);
+              write_miss(a, off, tr.fetches);
             }
           }
         }
@@ -473,7 +588,7 @@ __global__ void __launch_bounds__(256, kMinBlocks)
     for (;;) {
       int r = kContinue;
       uint32_t leaf = 0;
-#pragma unroll
+#pragma unroll 4
       for (int k = 0; k < kStepsPerVote; ++k)
         if ((mode == kPrimary || mode == kShadow) && r == kContinue)
           r = trace_step<kRef, kRing, kStaged, kLod>(sc, smw, nsm, stk, ring, tr,
@@ -483,42 +598,37 @@ __global__ void __launch_bounds__(256, kMinBlocks)
           // end of a shadow ray
           const bool sh = r == kHit;
           my_shadowed += sh ? 1u : 0u;
-          write_pixel(a, off, shade(attr, a, sh), hitw, ht, fp, tr.fetches, attr);
+          write_color(a, off, sh ? dark : lit, tr.fetches);
           mode = kIdle;
         } else if (r == kMiss) {
-          write_pixel(a, off, 0u, 0xFFFFFFFFu, 0.f, tr.fetches, 0u);
+          write_miss(a, off, tr.fetches);
           mode = kIdle;
         } else {
+          // everything but the colour is written now: the shadow ray carries
+          // two words along instead of the hit and its shading record (46
+          // registers at 5 blocks an SM, none spilled: 540 -> 526 us)
           ++my_hits;
-          hitw = ((kRef ? tr.node : __ldg(sc.orig_id + tr.node)) << 3) | (tr.ch ^ tr.df);
-          ht = max3f(tr.t.x1, tr.t.y1, tr.t.z1);
-          fp = tr.fetches;
-          attr = make_uint4(0u, 0u, 0u, 0u);
+          const uint32_t hitw = hit_word<kRef>(sc, tr, leaf);
+          const float ht = max3f(tr.t.x1, tr.t.y1, tr.t.z1);
+          uint4 attr = make_uint4(0u, 0u, 0u, 0u);
           if (leaf < sc.n_attrs)
             attr = load_shading<kRef>(sc, leaf);
           else
             err |= YV_DEV_ERR_POOL;
+          write_primary(a, off, hitw, ht, tr.fetches, attr);
+          lit = shade(attr, a, false);
           mode = kIdle;
           if (a.shadows) {
-            // shadow ray: the hit point moved half a leaf out through the entry face
+            dark = shade(attr, a, true);
             float o[3];
-            o[0] = __fadd_rn(a.pos[0], __fmul_rn(dx, ht));
-            o[1] = __fadd_rn(a.pos[1], __fmul_rn(dy, ht));
-            o[2] = __fadd_rn(a.pos[2], __fmul_rn(dz, ht));
-            int e = 0;
-            float m = tr.t.x1;
-            if (tr.t.y1 > m) { e = 1; m = tr.t.y1; }
-            if (tr.t.z1 > m) e = 2;
-            const float half = __int_as_float((127 - (tr.level + 2)) << 23);
-            const float d_off = ((tr.df >> e) & 1u) ? half : -half;
-            o[e] = __fadd_rn(o[e], d_off);
-            if (begin_trace(sc, o[0], o[1], o[2], a.light_ray[0], a.light_ray[1],
-                            a.light_ray[2], tr, err))
+            shadow_origin(a, tr, dx, dy, dz, ht, o);
+            if (begin_trace<kRef, kStaged>(sc, smw, nsm, o[0], o[1], o[2], a.light_ray[0],
+                                           a.light_ray[1], a.light_ray[2], tr, err))
               mode = kShadow;
             else
-              write_pixel(a, off, shade(attr, a, false), hitw, ht, fp, tr.fetches, attr);
+              write_color(a, off, lit, tr.fetches);
           } else {
-            write_pixel(a, off, shade(attr, a, false), hitw, ht, fp, 0u, attr);
+            write_color(a, off, lit, 0u);
           }
         }
       }

@@ -14,18 +14,27 @@
 // Device layout of the SVO node pool.
 //
 // The reference pool is an array of 40-byte VoxNode records read through a
-// 1D texture (reaction/report/main.tex:36-67).  On the device each node is
-// re-laid as one 32-byte, 32-byte-aligned record of 8 child words, so a node
-// is exactly one L2 sector (a traversal step reads the word it tests).  The leaf /
-// null information of `flags` is folded into the words:
+// 1D texture (reaction/report/main.tex:36-67).  On the device a traversal
+// reads one 8-byte record per node it enters, kept in registers while the
+// ray is in the node:
+//   .x  record of the first node child; the node children of a node are
+//       consecutive in child order
+//   .y  a nibble per child, child c in bits 28 - 4 c and up :
+//       0..7 a node, record .x + this; 8 null; 12 a leaf
+// and, only at a hit, the node's 8-byte cold record {caller node id, index of
+// its first leaf}; a node's leaves are consecutive too (leaf_attr maps a leaf
+// index to its attribute where the pool does not already number them so).
+// Records are breadth-first from the root, so the top levels come first.
+// A node that several parents share has one record per parent, all pointing
+// at the one run of its children.
+//
+// The traversal of a caller's VoxNode pool folds its flags into child words:
 //   word & YV_DW_LEAF  -> leaf, low 31 bits = VoxData (leaf attribute index)
 //   word & YV_DW_NULL  -> null child (EmptyNode / FullNode)
-//   otherwise          -> device node index
-// Nodes are renumbered breadth-first from the root, so the top levels are the
-// first records (they are staged in shared memory); orig_id maps a device
-// index back to the caller's node id for the hit output.
+//   otherwise          -> node index
 // ---------------------------------------------------------------------------
 constexpr uint32_t YV_DW_LEAF = 0x80000000u;
+constexpr uint32_t YV_CODE_NULL = 8u, YV_CODE_LEAF = 12u;
 constexpr uint32_t YV_DW_NULL = 0x40000000u;
 constexpr int YV_MAX_DEPTH = 16;            // node levels a pool may have
 constexpr uint32_t YV_MAX_DEVICE_NODES = 0x1FFFFFFFu;  // hit word = id<<3|c
@@ -48,10 +57,13 @@ namespace yv {
 
 // Breadth-first device re-layout of a reference pool (see above).
 struct DeviceLayout {
-  std::vector<uint32_t> words;     // 8 per node
-  std::vector<uint32_t> orig_id;   // device index -> caller node id
-  uint32_t root_word = YV_DW_NULL; // device word of the root
-  int depth = 0;                   // node levels (root = level 0)
+  std::vector<uint32_t> nodes;      // 2 per record: first node child, child codes
+  std::vector<uint32_t> cold;       // 2 per record: caller node id, first leaf
+  std::vector<uint32_t> leaf_attr;  // attribute of each leaf; empty: its index
+  uint32_t n_unique = 0;            // nodes reachable from the root
+  uint32_t root_word = YV_DW_NULL;  // record of the root, or YV_DW_NULL
+  int depth = 0;                    // node levels (root = level 0)
+  size_t records() const { return nodes.size() / 2; }
 };
 
 // Validates and converts; returns YV_OK or YV_ERR_BAD_POOL.
@@ -88,10 +100,10 @@ int hardware_threads();
 
 // Scenes built on the device (api.cpp): renderer_scene_buffers waits for
 // the renderer's last frame and returns its (reused or grown) buffers for nn
-// node records (8 child words, id) and na 16-byte shading records;
-// renderer_commit_scene then makes them the current scene.
-yv_status renderer_scene_buffers(yv_renderer* r, uint32_t nn, uint32_t na, uint32_t** words,
-                                 uint32_t** orig, void** attrs);
+// node records (8 bytes and their 8-byte cold records) and na 16-byte shading
+// records; renderer_commit_scene then makes them the current scene.
+yv_status renderer_scene_buffers(yv_renderer* r, uint32_t nn, uint32_t na, uint2** nodes,
+                                 uint2** cold, void** attrs);
 void renderer_commit_scene(yv_renderer* r, uint32_t nn, uint32_t na, uint32_t root_word);
 
 // A host brick volume from parts built on the device (volume_host.cpp):

@@ -10,8 +10,11 @@ namespace yv {
 
 // Device copy of an SVO scene (layout described in yv_internal.h).
 struct SvoDeviceScene {
-  const uint4* nodes = nullptr;       // 2 x uint4 (8 child words) per node
-  const uint32_t* orig_id = nullptr;  // device index -> caller node id
+  // 8-byte node records {first node child, child codes}; caller VoxNode pools: the
+  // 40-byte VoxNodes
+  const void* nodes = nullptr;
+  const uint2* cold = nullptr;          // {caller node id, first leaf} per record
+  const uint32_t* leaf_attr = nullptr;  // leaf -> attribute, or null: the same index
   // library layout: 16-byte shading records {RGBA8, unit normal xyz fp32};
   // caller VoxNode pools: the caller's yv_leaf_attr (8 bytes)
   const void* attrs = nullptr;
