@@ -84,3 +84,28 @@ def test_shared_nodes_and_attributes(oracle, yoxel_mod, kind, staged):
         todo += [int(c) for k, c in enumerate(nodes[i]["child"])
                  if not (nodes[i]["flags"] >> k) & 1 and not c & EMPTY]
     assert r.device_scene_info()[0] == len(seen)
+
+
+# frames around the sizes where a warp takes 8, 16 or 32 rays (from 8 rays a
+# warp on 152 SMs x 3 blocks x 8 warps: 29184 and 58368 ray ids), partial tiles
+@pytest.mark.parametrize("size", [(1, 1), (7, 3), (9, 5), (160, 120), (216, 136), (251, 233),
+                                  (333, 175), (640, 95)])
+@pytest.mark.parametrize("shadows", [False, True])
+def test_small_frames(oracle, yoxel_mod, size, shadows):
+    scene = yoxel_mod.SVOScene.spheres(6, 40, 2.0, 8.0, 77)
+    pos, view = camera_for()
+    w, h = size
+    r = yoxel_mod.Renderer()
+    r.SetScene(scene)
+    r.SetViewPos(pos)
+    r.SetViewDir(view)
+    r.SetResolution(w, h)
+    r.SetFOV(60.0)
+    r.SetLight(LIGHT, 0.15, 0.85, shadows)
+    out = r.render_outputs()
+    ref = oracle.svo_render(scene.nodes_u32, scene.root, scene.attrs_u8, pos, view, [0, 0, 1],
+                            60.0, w, h, LIGHT, shadows=shadows)
+    for k in ("hit", "rgba", "fetches", "shadow_fetches"):
+        np.testing.assert_array_equal(out[k].cpu().numpy().view(np.uint32), ref[k], err_msg=k)
+    np.testing.assert_array_equal(out["hit_t"].cpu().numpy(), ref["hit_t"])
+    assert out["stats"]["primary_rays"] == w * h

@@ -55,6 +55,18 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
 
 cudaError_t scratch_free(void* p, cudaStream_t s) { return p ? cudaFreeAsync(p, s) : cudaSuccess; }
 
+// Rays a warp takes at a time: 32, or 16 or 8 when the frame's rays so split
+// still fit the resident warps.  A small frame ends with its slowest warp,
+// and a warp runs every branch that any of its rays takes: fewer rays to a
+// warp is a shorter chain (160x120, 256^3 spheres: 60 us at 32 rays, 52 at 8;
+// 4 rays gained nothing more).  A frame that fills the GPU keeps 32.
+uint32_t frame_lanes(const SvoFrameArgs& a, uint64_t warps) {
+  const uint64_t ids = a.id_end - a.id_begin;
+  uint32_t lanes = 32;
+  while (lanes > 8u && ids <= warps * (lanes / 2)) lanes /= 2;
+  return lanes;
+}
+
 template <int kMinBlocks, bool kStaged, bool kLod = false, bool kRef = false>
 static cudaError_t launch_with(const SvoDeviceScene& sc, const SvoFrameArgs& a, int bt,
                                uint32_t nsm, uint32_t refill, int per_sm, cudaStream_t stream) {
@@ -84,7 +96,8 @@ static cudaError_t launch_with(const SvoDeviceScene& sc, const SvoFrameArgs& a, 
   const int grid = device_sm_count() * (per_sm > 0 && per_sm < resident ? per_sm : resident);
   e = cudaMemsetAsync(a.counters, 0, kSvoCounterWords * sizeof(uint32_t), stream);
   if (e != cudaSuccess) return e;
-  kern<<<grid, bt, smem, stream>>>(sc, a, nsm, refill);
+  kern<<<grid, bt, smem, stream>>>(sc, a, nsm, refill,
+                                   frame_lanes(a, (uint64_t)grid * (uint64_t)(bt / 32)));
   return cudaGetLastError();
 }
 

@@ -125,7 +125,8 @@ extern "C" yv_status yv_render_svo_noalloc(const yv_vox_node* nodes, uint32_t co
   if (e == cudaSuccess)
     e = cudaMemsetAsync(scratch, 0, kSvoCounterWords * sizeof(uint32_t), s);
   if (e == cudaSuccess) {
-    kern<<<device_sm_count() * resident, 256, kSmem, s>>>(sc, a, 0u, 32u);
+    const int grid = device_sm_count() * resident;
+    kern<<<grid, 256, kSmem, s>>>(sc, a, 0u, 32u, frame_lanes(a, (uint64_t)grid * (256 / 32)));
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {

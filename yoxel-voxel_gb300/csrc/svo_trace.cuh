@@ -515,9 +515,12 @@ __device__ __forceinline__ void shadow_origin(const SvoFrameArgs& a, const Trace
 // so the default is unstaged and nsm = 0).
 // Dynamic shared memory = 8 B x nsm staged nodes + 1 KB x kRing per warp.
 // kLod: level-of-detail cut-off (a.lod_coef, sc.node_data; library layout).
+// lanes: rays a warp takes at a time (the other lanes stay idle), for frames
+// too small to fill the GPU (frame_lanes).
 template <int kMinBlocks, bool kRef, int kRing, bool kStaged, bool kLod = false>
 __global__ void __launch_bounds__(256, kMinBlocks)
-    svo_frame_kernel(SvoDeviceScene sc, SvoFrameArgs a, uint32_t nsm, uint32_t refill_min) {
+    svo_frame_kernel(SvoDeviceScene sc, SvoFrameArgs a, uint32_t nsm, uint32_t refill_min,
+                     uint32_t lanes) {
   extern __shared__ uint4 smem[];
   // the block's deadline under a frame budget (held in shared memory, not
   // in a register of the traversal)
@@ -539,7 +542,7 @@ __global__ void __launch_bounds__(256, kMinBlocks)
   const uint32_t n_ids = a.id_end;
   uint32_t err = 0, my_hits = 0, my_shadowed = 0;
 
-  uint32_t mode = kIdle, off = 0;
+  uint32_t mode = lane < lanes ? kIdle : kDone, off = 0;
   Trace tr;
   float dx = 0.f, dy = 0.f, dz = 0.f;
   // colours of the pixel whose shadow ray is under way, lit and in shadow
@@ -565,8 +568,10 @@ __global__ void __launch_bounds__(256, kMinBlocks)
           mode = kDone;
         } else {
           const uint32_t tile = id >> 5, w = id & 31u;
-          const int x = (int)((tile % tiles_x) * 8u + (w & 7u));
-          const int y = (int)((tile / tiles_x) * 4u + (w >> 3));
+          // a tile's two 4x4 halves, each in rows of 4: any 4, 8 or 16
+          // consecutive ids are neighbouring pixels
+          const int x = (int)((tile % tiles_x) * 8u + ((w & 3u) | ((w >> 2) & 4u)));
+          const int y = (int)((tile / tiles_x) * 4u + ((w >> 2) & 3u));
           if (x < a.width && y < a.height) {
             off = (uint32_t)y * (uint32_t)a.width + (uint32_t)x;
             pixel_dir(a, x, y, dx, dy, dz);

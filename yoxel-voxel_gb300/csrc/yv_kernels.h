@@ -75,6 +75,9 @@ cudaError_t launch_svo_frame(const SvoDeviceScene& sc, const SvoFrameArgs& a,
                              const LaunchCfg& cfg, cudaStream_t stream,
                              int* launches);
 
+// Rays a warp of the frame kernel takes at a time when `warps` are resident.
+uint32_t frame_lanes(const SvoFrameArgs& a, uint64_t warps);
+
 // Number of SMs of the current device (cached per device).
 int device_sm_count();
 
