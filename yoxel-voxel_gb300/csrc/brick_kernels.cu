@@ -7,25 +7,26 @@
 namespace yv {
 namespace {
 
-// Register budget of the adjoint (resident blocks of 256 per SM): its 16
+// Threads of a march block: half of a 16x16-pixel square.  A block holds its
+// registers until its slowest warp ends, so smaller blocks keep more warps at
+// work: 64-camera training step 10.04 ms at 256 threads, 9.66 at 128, 9.79 at
+// 64; 1024^2 frame of a 512^3 volume 740 / 704 / 719 us.
+constexpr int kMarchThreads = 128;
+// Register budget of the adjoint (resident warps per SM / 8): its 16
 // per-lane gradient accumulators live in registers (a shared-memory copy
 // measured 1.25x slower).
 constexpr int kBackwardMinBlocks = 3;
-// Register budget of the forward march per lattice format: the fp16 +
-// 8-bit colour formats (0, 3) run at 3 resident blocks (74 registers for the
-// 8-byte format: 1.19 ms on the 1024^2 frame of a 512^3 volume, against 1.26
-// ms at 4 blocks / 64 registers and 1.43 ms at 5 / 48 with spills); the fp32
-// formats (1, 2) at 4 (the 64-camera 128^3 forward: 3.19 ms at 4 blocks,
-// 3.29 ms at 3).  Measured while the grid nodes were staged in shared
-// memory; re-measured for the 8-byte format without staging: 904 / 843 /
-// 754 Mrays/s at 3 / 4 / 5 blocks.
+// Register budget of the forward march per lattice format (resident warps
+// per SM / 8): 3 for the fp16 + 8-bit colour formats (0, 3), 4 for the fp32
+// formats (1, 2).  1024^2 frame of a 512^3 volume, 8-byte format: 740 us at 3,
+// 764 at 4; 64-camera fp32 training step 10.04 ms at 4, 10.13 at 3.
 template <int P>
 struct ForwardBlocks {
   static constexpr int value = (P == 0 || P == 3) ? 3 : 4;
 };
 
 // tile mapping: warp w of the grid -> 8x4 pixel tile of one camera image;
-// the 8 warps of a block take a 2x4-tile (16x16-pixel) square
+// 8 consecutive tiles are a 2x4-tile (16x16-pixel) square
 __host__ __device__ __forceinline__ uint32_t tile_ids(const VolumeArgs& a) {
   const uint32_t tx = (uint32_t)((a.width + 7) >> 3), ty = (uint32_t)((a.height + 3) >> 2);
   return (uint32_t)a.ncams * ((tx + 1) >> 1) * ((ty + 3) >> 2) * 8u;
@@ -57,14 +58,14 @@ __device__ __forceinline__ uint32_t rgba8_of(float r, float g, float b, float al
   return out;
 }
 
-// kMinBlocks: resident blocks of 256 per SM the register allocation is
-// sized for.
+// kMinBlocks: resident warps per SM / 8 the register allocation is sized for.
+// Bound by instruction issue.  On the 1024^2 frame of a 512^3 volume (8-byte
+// format) 876 -> 740 us from the cell found by one round-down add instead of
+// a conversion and clamps, the fraction clamped by the add's saturation, and
+// the half decoded by one conversion; 704 us with blocks of 128 threads.
 // kSkip: the pool carries a cell occupancy mask (a learnable pool does not).
 template <int P, int kMinBlocks, bool kSkip>
-__global__ void __launch_bounds__(256, kMinBlocks) volume_forward_kernel(VolumeArgs a) {
-  // grid nodes are read through L1 (see prefer_l1)
-  const uint32_t* sg = nullptr;
-  const uint32_t nsg = 0;
+__global__ void __launch_bounds__(kMarchThreads, 2 * kMinBlocks) volume_forward_kernel(VolumeArgs a) {
   // the launch's tiles (a range of them for a frame split across GPUs)
   const uint32_t n_tiles = a.tile_end ? a.tile_end : tile_ids(a);
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -77,7 +78,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) volume_forward_kernel(VolumeA
     pixel_ray(a.cam[cam], x, y, o, d);
     NoVis nv;
     RayOut r;
-    march<P, NoVis, true, kSkip>(a.v, sg, nsg, o, d, nv, r);
+    march<P, NoVis, true, kSkip>(a.v, o, d, nv, r);
     bad |= r.bad;
     const size_t off = ((size_t)cam * a.height + (size_t)y) * a.width + (size_t)x;
     if (a.rgba) reinterpret_cast<float4*>(a.rgba)[off] = make_float4(r.c[0], r.c[1], r.c[2], r.a);
@@ -136,8 +137,7 @@ struct GradVis {
       atomicAdd(a->grad_packed + base + corner_offset(j),
                 make_float4(fmul(g[0], gw[j]), fmul(g[1], gw[j]), fmul(g[2], gw[j]), gd[j]));
   }
-  __device__ __forceinline__ void operator()(const SampleCtx& s, float T, float w, float, float,
-                                             float, float) {
+  __device__ __forceinline__ void operator()(const SampleCtx& s, float T, float w) {
     const float gc = ffma(g[2], s.col[2], ffma(g[1], s.col[1], ffma(g[0], s.col[0], g[3])));
     const float ds = sample_dsigma(a, gc, gout, gb, s, T, w);
     gb = ffma(w, gc, gb);
@@ -159,12 +159,10 @@ struct GradVis {
   }
 };
 
-// kMinBlocks: register budget (resident blocks of 256 per SM).
+// kMinBlocks: register budget (resident warps per SM / 8).
 template <int P, int kMinBlocks>
 // grid nodes are read through L1 (see prefer_l1)
-__global__ void __launch_bounds__(256, kMinBlocks) volume_backward_kernel(VolumeArgs a) {
-  const uint32_t* sg = nullptr;
-  const uint32_t nsg = 0;
+__global__ void __launch_bounds__(kMarchThreads, 2 * kMinBlocks) volume_backward_kernel(VolumeArgs a) {
   const uint32_t n_tiles = tile_ids(a);
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   bool bad = false;
@@ -184,7 +182,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) volume_backward_kernel(Volume
     gv.gout = ffma(g4.w, o4.w, ffma(g4.z, o4.z, ffma(g4.y, o4.y, fmul(g4.x, o4.x))));
     gv.init();
     RayOut r;
-    march<P, GradVis, false>(a.v, sg, nsg, o, d, gv, r);
+    march<P, GradVis, false>(a.v, o, d, gv, r);
     gv.flush();
     bad |= r.bad;
   }
@@ -224,7 +222,7 @@ __global__ void brick_bits_kernel(VolumeView v, uint32_t* bits, uint32_t nwords)
   bool set = false;
   if (ci < n) {
     const int cell[3] = {(int)(ci % nb), (int)((ci / nb) % nb), (int)(ci / (nb * nb))};
-    set = lookup(v, nullptr, 0u, cell) != -1;
+    set = lookup(v, cell) != -1;
   }
   const uint32_t word = __ballot_sync(0xFFFFFFFFu, set);
   if ((threadIdx.x & 31u) == 0) bits[w] = word;
@@ -316,34 +314,34 @@ uint32_t volume_tiles_per_camera(int width, int height) {
 cudaError_t launch_volume_forward(const VolumeArgs& a, cudaStream_t s) {
   const uint32_t end = a.tile_end ? a.tile_end : tile_ids(a);
   const uint32_t tiles = end > a.tile_begin ? end - a.tile_begin : 0u;
-  const uint32_t blocks = (tiles + 7) / 8;
+  const uint32_t blocks = (tiles + kMarchThreads / 32 - 1) / (kMarchThreads / 32);
   if (blocks == 0) return cudaSuccess;
   prefer_l1();
   const bool skip = a.v.cell_mask != nullptr;
   switch (a.v.precision) {
     case 0:
       if (skip)
-        volume_forward_kernel<0, ForwardBlocks<0>::value, true><<<blocks, 256, 0, s>>>(a);
+        volume_forward_kernel<0, ForwardBlocks<0>::value, true><<<blocks, kMarchThreads, 0, s>>>(a);
       else
-        volume_forward_kernel<0, ForwardBlocks<0>::value, false><<<blocks, 256, 0, s>>>(a);
+        volume_forward_kernel<0, ForwardBlocks<0>::value, false><<<blocks, kMarchThreads, 0, s>>>(a);
       break;
     case 1:
       if (skip)
-        volume_forward_kernel<1, ForwardBlocks<1>::value, true><<<blocks, 256, 0, s>>>(a);
+        volume_forward_kernel<1, ForwardBlocks<1>::value, true><<<blocks, kMarchThreads, 0, s>>>(a);
       else
-        volume_forward_kernel<1, ForwardBlocks<1>::value, false><<<blocks, 256, 0, s>>>(a);
+        volume_forward_kernel<1, ForwardBlocks<1>::value, false><<<blocks, kMarchThreads, 0, s>>>(a);
       break;
     case 2:
       if (skip)
-        volume_forward_kernel<2, ForwardBlocks<2>::value, true><<<blocks, 256, 0, s>>>(a);
+        volume_forward_kernel<2, ForwardBlocks<2>::value, true><<<blocks, kMarchThreads, 0, s>>>(a);
       else
-        volume_forward_kernel<2, ForwardBlocks<2>::value, false><<<blocks, 256, 0, s>>>(a);
+        volume_forward_kernel<2, ForwardBlocks<2>::value, false><<<blocks, kMarchThreads, 0, s>>>(a);
       break;
     case 3:
       if (skip)
-        volume_forward_kernel<3, ForwardBlocks<3>::value, true><<<blocks, 256, 0, s>>>(a);
+        volume_forward_kernel<3, ForwardBlocks<3>::value, true><<<blocks, kMarchThreads, 0, s>>>(a);
       else
-        volume_forward_kernel<3, ForwardBlocks<3>::value, false><<<blocks, 256, 0, s>>>(a);
+        volume_forward_kernel<3, ForwardBlocks<3>::value, false><<<blocks, kMarchThreads, 0, s>>>(a);
       break;
     default: return cudaErrorInvalidValue;
   }
@@ -352,14 +350,14 @@ cudaError_t launch_volume_forward(const VolumeArgs& a, cudaStream_t s) {
 
 cudaError_t launch_volume_backward(const VolumeArgs& a, cudaStream_t s) {
   const uint32_t tiles = tile_ids(a);
-  const uint32_t blocks = (tiles + 7) / 8;
+  const uint32_t blocks = (tiles + kMarchThreads / 32 - 1) / (kMarchThreads / 32);
   if (blocks == 0) return cudaSuccess;
   prefer_l1();
   // only fp32 (learnable) volumes have an adjoint
   if (a.v.precision == 1)
-    volume_backward_kernel<1, kBackwardMinBlocks><<<blocks, 256, 0, s>>>(a);
+    volume_backward_kernel<1, kBackwardMinBlocks><<<blocks, kMarchThreads, 0, s>>>(a);
   else if (a.v.precision == 2)
-    volume_backward_kernel<2, kBackwardMinBlocks><<<blocks, 256, 0, s>>>(a);
+    volume_backward_kernel<2, kBackwardMinBlocks><<<blocks, kMarchThreads, 0, s>>>(a);
   else
     return cudaErrorInvalidValue;
   return cudaGetLastError();

@@ -58,19 +58,6 @@ __device__ __forceinline__ float byte_f(uint32_t v, int k) {
   return __fsub_rn(__uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440u + (uint32_t)k)),
                    8388608.f);
 }
-// 0 <= n < 2^23 as a float (exact).
-__device__ __forceinline__ float small_int_f(int n) {
-  return __fsub_rn(__uint_as_float(0x4B000000u | (uint32_t)n), 8388608.f);
-}
-// Finite binary16 in the low 16 bits of h as a float: the half's exponent
-// and mantissa bits placed in a float (a subnormal for every half) and
-// scaled by 2^112, exact for normal and subnormal halves alike.  The fp16
-// lattice formats hold finite values only (the upload saturates).
-__device__ __forceinline__ float half_bits_f(uint32_t h) {
-  const uint32_t m = ((h & 0x7FFFu) << 13) | ((h & 0x8000u) << 16);
-  return __fmul_rn(__uint_as_float(m), __uint_as_float(0x77800000u));  // x 2^112
-}
-
 template <int P>
 struct Voxel;
 
@@ -126,7 +113,7 @@ struct Voxel<3> {
   __device__ static __forceinline__ void corner(const VolumeView& a, uint32_t i, float& d,
                                                 float* c) {
     const uint2 v = __ldg(static_cast<const uint2*>(a.albedo) + i);
-    d = half_bits_f(v.x);
+    d = __half2float(__ushort_as_half((unsigned short)(v.x & 0xFFFFu)));
     c[0] = byte_f(v.x, 2);
     c[1] = byte_f(v.x, 3);
     c[2] = byte_f(v.y, 0);
@@ -135,9 +122,6 @@ struct Voxel<3> {
 
 struct SampleCtx {
   uint32_t base;  // brick*729 + corner-000 lattice index
-  int brick;      // brick and brick-local corner-000 lattice coordinates
-  int cell[3];
-  float f[3];     // fractional position inside the trilinear cell
   float w[8];     // trilinear weights, corner j: bit0 +x, bit1 +y, bit2 +z
   float sigma, alpha;
   float col[3];
@@ -172,30 +156,37 @@ __device__ __forceinline__ void sample_coord(float t, float D, float Lh, float L
   l = fadd(p, Lh);
 }
 
+// floor of a lattice coordinate clamped to cell 0..7 as 2^23 + k, the integer
+// k in its low bits (0x4B000000 | k): one add that rounds down, in place of a
+// conversion (quarter rate) and integer clamps.
+__device__ __forceinline__ float cell_of(float l) {
+  return __fadd_rd(fminf(fmaxf(l, 0.f), 7.f), 8388608.f);
+}
+
+// Whether the cell kb (cell_of) of brick b has its bit in the cell occupancy
+// mask: bit (y & 3) * 8 + x of word z * 2 + (y >> 2).  The constants that
+// cell_of adds vanish in the shift (modulo 32) and cancel in the word index.
+__device__ __forceinline__ bool cell_marked(const VolumeView& a, int b, const float* kb) {
+  const uint32_t x = __float_as_uint(kb[0]), y = __float_as_uint(kb[1]),
+                 z = __float_as_uint(kb[2]);
+  const uint32_t w = (uint32_t)b * 16u - 0x4B000000u * 2u - (0x4B000000u >> 2) + z * 2u + (y >> 2);
+  return (__ldg(a.cell_mask + w) >> ((y * 8u + x) & 31u)) & 1u;
+}
+
 // l + e: brick-local lattice coordinates of the sample (sample_coord), in
-// [0, 8].
+// [0, 8]; kb its cell (cell_of).
 template <int P>
 __device__ __forceinline__ void eval_sample(const VolumeView& a, int b, const float* l,
-                                            const float* e, SampleCtx& s) {
-  int i0[3];
+                                            const float* e, const float* kb, SampleCtx& s) {
   float f[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    int k = __float2int_rd(l[i]);
-    k = k < 0 ? 0 : (k > 7 ? 7 : k);
-    float fi = fadd(fsub(l[i], small_int_f(k)), e[i]);
-    fi = fi < 0.f ? 0.f : (fi > 1.f ? 1.f : fi);
-    i0[i] = k;
-    f[i] = fi;
+    // saturate: a fraction a rounding outside [0, 1] is clamped
+    f[i] = __saturatef(fadd(fsub(l[i], fsub(kb[i], 8388608.f)), e[i]));
   }
-  s.base = (uint32_t)b * (uint32_t)kL3 + (uint32_t)((i0[2] * kL + i0[1]) * kL + i0[0]);
-  s.brick = b;
-  s.cell[0] = i0[0];
-  s.cell[1] = i0[1];
-  s.cell[2] = i0[2];
-  s.f[0] = f[0];
-  s.f[1] = f[1];
-  s.f[2] = f[2];
+  // k + 0x4B000000 in each coordinate: the constants cancel modulo 2^32
+  s.base = (uint32_t)b * (uint32_t)kL3 - 0x4B000000u * 91u + __float_as_uint(kb[2]) * 81u +
+           __float_as_uint(kb[1]) * 9u + __float_as_uint(kb[0]);
   const float gx = fsub(1.f, f[0]), gy = fsub(1.f, f[1]), gz = fsub(1.f, f[2]);
   const float w00 = fmul(gx, gy), w10 = fmul(f[0], gy), w01 = fmul(gx, f[1]),
               w11 = fmul(f[0], f[1]);
@@ -226,18 +217,16 @@ __device__ __forceinline__ void eval_sample(const VolumeView& a, int b, const fl
 }
 
 // Tree descent for brick cell `cell` (ntree/ntree/nodes.h:56-99 offsets).
-// Grid nodes below nsg come from sg (a shared-memory copy; the kernels pass
-// none and read every node through L1).  Returns brick id, -1 if empty,
-// -2 if the pool is malformed.
-__device__ __forceinline__ int lookup(const VolumeView& a, const uint32_t* sg, uint32_t nsg,
-                                      const int* cell) {
+// Every node is read through L1.  Returns brick id, -1 if empty, -2 if the
+// pool is malformed.
+__device__ __forceinline__ int lookup(const VolumeView& a, const int* cell) {
   uint32_t node = 0;
   for (int lev = 0; lev < a.levels; ++lev) {
     const int sh = 2 * (a.levels - 1 - lev);
     const uint32_t c = (uint32_t)((((cell[2] >> sh) & 3) * 4 + ((cell[1] >> sh) & 3)) * 4 +
                                   ((cell[0] >> sh) & 3));
     if (node >= a.ngrids) return -2;
-    const uint32_t ref = node < nsg ? sg[node * 64 + c] : __ldg(a.grids + (size_t)node * 64 + c);
+    const uint32_t ref = __ldg(a.grids + (size_t)node * 64 + c);
     if (ref & kEmpty) return -1;
     if (ref & kBrick) {
       const uint32_t b = ref & 0x3FFFFFFFu;
@@ -257,118 +246,149 @@ struct RayOut {
   bool bad;
 };
 
-// One ray; `Vis` is called per sample with (sample, T, T alpha, A and C
-// before the sample).
-// kColor = false (the adjoint's replay): the composited colour is not
-// accumulated (the visitor tracks what it needs; r.c stays 0).
-// kSkip: the forward passes over the samples of cells the pool's
-// cell_mask marks empty (compiled out for pools without one).
-template <int P, class Vis, bool kColor = true, bool kSkip = kColor>
-__device__ __forceinline__ void march(const VolumeView& a, const uint32_t* sg, uint32_t nsg,
-                                      const float* o, const float* d, Vis& vis, RayOut& r) {
-  r.c[0] = r.c[1] = r.c[2] = 0.f;
-  r.a = 0.f;
-  r.samples = 0;
-  r.bricks = 0;
-  r.bad = false;
-  float inv[3], t1[3], t2[3];
+// State of one ray's march: the DDA over brick cells and, inside an occupied
+// one, the run of its samples.
+// kLean keeps less of it alive for the adjoint's tighter register budget: the
+// step direction of an axis is the sign of inv (d is never 0), and the
+// lattice-space origin o S is recomputed (the same rounded product) at each
+// occupied cell.
+template <bool kLean>
+struct March {
+  float inv[3], D[3], Q[kLean ? 1 : 3];  // 1 / d; lattice-space direction, origin
+  int cell[3];
+  float t_in, t_out;
+  int e;  // exit axis of the current cell
+  // occupied cell: brick, its local origin as an exact pair, next sample
+  int b, k;
+  float Lh[3], Ll[3], t;
+};
+
+// Clips the ray to the unit cube; false: it misses.
+template <bool kLean>
+__device__ __forceinline__ bool march_begin(const VolumeView& a, const float* o, const float* d,
+                                            March<kLean>& m) {
+  float t1[3], t2[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    inv[i] = __fdiv_rn(1.f, d[i]);
-    const float lo = fmul(fsub(0.f, o[i]), inv[i]);
-    const float hi = fmul(fsub(1.f, o[i]), inv[i]);
+    m.inv[i] = __fdiv_rn(1.f, d[i]);
+    const float lo = fmul(fsub(0.f, o[i]), m.inv[i]);
+    const float hi = fmul(fsub(1.f, o[i]), m.inv[i]);
     t1[i] = lo < hi ? lo : hi;
     t2[i] = lo < hi ? hi : lo;
   }
   float t_enter = fmaxf(fmaxf(t1[0], t1[1]), t1[2]);
   const float t_exit = fminf(fminf(t2[0], t2[1]), t2[2]);
   if (t_enter < 0.f) t_enter = 0.f;
-  if (t_exit < 0.f || t_enter > t_exit) return;
-  const float h = a.cell_size;  // world size of a brick cell
-  // The replay (kColor = false) keeps less live state for its tighter
-  // register budget: the step direction of an axis is the sign of inv (d is
-  // never 0), and the lattice-space origin o S is recomputed (the same
-  // rounded product) at each occupied cell (cfg4 adjoint 7.10 -> 6.83 ms;
-  // the forward measured faster holding them).
-  int cell[3], step[3];
-  float Q[3], D[3];  // lattice-space origin and direction
+  if (t_exit < 0.f || t_enter > t_exit) return false;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const float q = __fdiv_rn(fadd(o[i], fmul(t_enter, d[i])), h);
+    const float q = __fdiv_rn(fadd(o[i], fmul(t_enter, d[i])), a.cell_size);
     int k = __float2int_rd(q);
-    k = k < 0 ? 0 : (k > a.nb - 1 ? a.nb - 1 : k);
-    cell[i] = k;
-    step[i] = d[i] > 0.f ? 1 : -1;
-    Q[i] = fmul(o[i], a.S);
-    D[i] = fmul(d[i], a.S);
+    m.cell[i] = k < 0 ? 0 : (k > a.nb - 1 ? a.nb - 1 : k);
+    if (!kLean) m.Q[i] = fmul(o[i], a.S);
+    m.D[i] = fmul(d[i], a.S);
   }
-  float t_in = t_enter;
+  m.t_in = t_enter;
+  return true;
+}
+
+// The current brick cell: its exit and what the tree holds there (brick id,
+// -1 empty, -2 malformed).
+template <bool kLean>
+__device__ __forceinline__ int march_cell(const VolumeView& a, const float* o, March<kLean>& m) {
+  float tx[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const bool up = m.inv[i] > 0.f;
+    const float plane = fmul((float)(up ? m.cell[i] + 1 : m.cell[i]), a.cell_size);
+    tx[i] = fmul(fsub(plane, o[i]), m.inv[i]);
+  }
+  // exit axis = first argmin (selects, no dynamic register indexing)
+  m.e = 0;
+  m.t_out = tx[0];
+  if (tx[1] < m.t_out) { m.e = 1; m.t_out = tx[1]; }
+  if (tx[2] < m.t_out) { m.e = 2; m.t_out = tx[2]; }
+  // the tree is descended only where the brick bitmap (if any) says a brick
+  // may be
+  const uint32_t ci =
+      ((uint32_t)m.cell[2] * (uint32_t)a.nb + (uint32_t)m.cell[1]) * (uint32_t)a.nb +
+      (uint32_t)m.cell[0];
+  if (a.brick_bits && !((__ldg(a.brick_bits + (ci >> 5)) >> (ci & 31u)) & 1u)) return -1;
+  return lookup(a, m.cell);
+}
+
+// Into the next brick cell; false: the ray leaves the volume.
+template <bool kLean>
+__device__ __forceinline__ bool march_next(const VolumeView& a, March<kLean>& m) {
+  m.t_in = m.t_out;
+  int ce;
+  if (m.e == 0) ce = (m.cell[0] += m.inv[0] > 0.f ? 1 : -1);
+  else if (m.e == 1) ce = (m.cell[1] += m.inv[1] > 0.f ? 1 : -1);
+  else ce = (m.cell[2] += m.inv[2] > 0.f ? 1 : -1);
+  return ce >= 0 && ce < a.nb;
+}
+
+// The samples of the occupied cell b: the brick-local origin Q - 8c as an
+// exact pair - the brick-local coordinate t D + (Q - 8c) in [0, 8] is formed
+// without the rounding of |Q| (sample_coord) - and the first sample.
+template <bool kLean>
+__device__ __forceinline__ void march_enter(const VolumeView& a, const float* o, int b,
+                                            March<kLean>& m) {
+  m.b = b;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    two_sum(kLean ? fmul(o[i], a.S) : m.Q[kLean ? 0 : i], -(float)(8 * m.cell[i]), m.Lh[i],
+            m.Ll[i]);
+  m.k = __float2int_ru(fmul(m.t_in, a.inv_dt));
+  m.t = fmul((float)m.k, a.dt);
+}
+
+// One ray; `Vis` is called per sample with (sample, T, T alpha).
+// kColor = false (the adjoint's replay): the composited colour is not
+// accumulated (the visitor tracks what it needs; r.c stays 0).
+// kSkip: the forward passes over the samples of cells the pool's
+// cell_mask marks empty (compiled out for pools without one).
+template <int P, class Vis, bool kColor = true, bool kSkip = kColor>
+__device__ __forceinline__ void march(const VolumeView& a, const float* o, const float* d,
+                                      Vis& vis, RayOut& r) {
+  r.c[0] = r.c[1] = r.c[2] = 0.f;
+  r.a = 0.f;
+  r.samples = 0;
+  r.bricks = 0;
+  r.bad = false;
+  March<!kColor> m;
+  if (!march_begin(a, o, d, m)) return;
   float A = 0.f, C0 = 0.f, C1 = 0.f, C2 = 0.f;
   for (int guard = 0; guard < 4 * 4096; ++guard) {
-    float tx[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const bool up = kColor ? d[i] > 0.f : inv[i] > 0.f;
-      const float plane = fmul((float)(up ? cell[i] + 1 : cell[i]), h);
-      tx[i] = fmul(fsub(plane, o[i]), inv[i]);
-    }
-    // exit axis = first argmin (selects, no dynamic register indexing)
-    int e = 0;
-    float t_out = tx[0];
-    if (tx[1] < t_out) { e = 1; t_out = tx[1]; }
-    if (tx[2] < t_out) { e = 2; t_out = tx[2]; }
-    int b = -1;
-    {
-      // the tree is descended only where the brick bitmap (if any) says a
-      // brick may be
-      const uint32_t ci =
-          ((uint32_t)cell[2] * (uint32_t)a.nb + (uint32_t)cell[1]) * (uint32_t)a.nb +
-          (uint32_t)cell[0];
-      if (!a.brick_bits || ((__ldg(a.brick_bits + (ci >> 5)) >> (ci & 31u)) & 1u))
-        b = lookup(a, sg, nsg, cell);
-    }
+    const int b = march_cell(a, o, m);
     if (b == -2) {
       r.bad = true;
       break;
     }
     if (b >= 0) {
       ++r.bricks;
-      // the brick-local origin Q - 8c as an exact pair: the brick-local
-      // coordinate t D + (Q - 8c) in [0, 8] is formed without the rounding
-      // of |Q| (sample_coord)
-      float Lh[3], Ll[3];
+      march_enter(a, o, b, m);
+      for (int it = 0; it < 1 << 16; ++it, ++m.k, m.t = fmul((float)m.k, a.dt)) {
+        if (!(m.t < m.t_out)) break;
+        float lc[3], le[3], kb[3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-        two_sum(kColor ? Q[i] : fmul(o[i], a.S), -(float)(8 * cell[i]), Lh[i], Ll[i]);
-      int k = __float2int_ru(fmul(t_in, a.inv_dt));
-      for (int it = 0; it < 1 << 16; ++it, ++k) {
-        const float t = fmul((float)k, a.dt);
-        if (!(t < t_out)) break;
-        float lc[3], le[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) sample_coord(t, D[i], Lh[i], Ll[i], lc[i], le[i]);
-        if (kColor && kSkip && a.cell_mask) {
+        for (int i = 0; i < 3; ++i) {
+          sample_coord(m.t, m.D[i], m.Lh[i], m.Ll[i], lc[i], le[i]);
+          kb[i] = cell_of(lc[i]);
+        }
+        if (kColor && kSkip && a.cell_mask && !cell_marked(a, b, kb)) {
           // a cell whose 8 corners are all zero has sigma = 0, alpha = 0:
           // the sample adds exactly nothing (C, A unchanged), so the
           // forward passes over it; the replay of the adjoint, whose
           // density gradient reaches such samples, takes every sample
-          int kc[3];
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            const int kk = __float2int_rd(lc[i]);
-            kc[i] = kk < 0 ? 0 : (kk > 7 ? 7 : kk);
-          }
-          const uint32_t mw = __ldg(a.cell_mask + (size_t)b * 16u + (uint32_t)(kc[2] * 2 + (kc[1] >> 2)));
-          if (!((mw >> (((kc[1] & 3) << 3) | kc[0])) & 1u)) {
-            ++r.samples;
-            continue;
-          }
+          ++r.samples;
+          continue;
         }
         SampleCtx s;
-        eval_sample<P>(a, b, lc, le, s);
+        eval_sample<P>(a, b, lc, le, kb, s);
         const float T = fsub(1.f, A);
         const float w = fmul(T, s.alpha);
-        vis(s, T, w, A, C0, C1, C2);
+        vis(s, T, w);
         if (kColor) {
           C0 = ffma(w, s.col[0], C0);
           C1 = ffma(w, s.col[1], C1);
@@ -379,12 +399,7 @@ __device__ __forceinline__ void march(const VolumeView& a, const uint32_t* sg, u
         if (A > 0.99f) goto done;
       }
     }
-    t_in = t_out;
-    int ce;
-    if (e == 0) ce = (cell[0] += kColor ? step[0] : (inv[0] > 0.f ? 1 : -1));
-    else if (e == 1) ce = (cell[1] += kColor ? step[1] : (inv[1] > 0.f ? 1 : -1));
-    else ce = (cell[2] += kColor ? step[2] : (inv[2] > 0.f ? 1 : -1));
-    if (ce < 0 || ce >= a.nb) break;
+    if (!march_next(a, m)) break;
   }
 done:
   r.c[0] = C0;
@@ -394,8 +409,7 @@ done:
 }
 
 struct NoVis {
-  __device__ __forceinline__ void operator()(const SampleCtx&, float, float, float, float, float,
-                                             float) {}
+  __device__ __forceinline__ void operator()(const SampleCtx&, float, float) {}
 };
 
 __device__ __forceinline__ void pixel_ray(const CamBasis& c, int x, int y, float* o, float* d) {
