@@ -31,16 +31,20 @@ __host__ __device__ __forceinline__ uint32_t tile_ids(const VolumeArgs& a) {
   const uint32_t tx = (uint32_t)((a.width + 7) >> 3), ty = (uint32_t)((a.height + 3) >> 2);
   return (uint32_t)a.ncams * ((tx + 1) >> 1) * ((ty + 3) >> 2) * 8u;
 }
-__device__ __forceinline__ bool ray_of_thread(const VolumeArgs& a, uint32_t tile, int& cam,
-                                              int& x, int& y) {
+// `sub`: part sub % (32 / a.lanes) of tile sub / (32 / a.lanes), a.lanes rays
+// of the tile's two 4x4 halves (each in rows of 4), one per lane from lane 0.
+__device__ __forceinline__ bool ray_of_thread(const VolumeArgs& a, uint32_t sub, int& cam, int& x,
+                                              int& y) {
   const uint32_t tx = (uint32_t)((a.width + 7) >> 3), ty = (uint32_t)((a.height + 3) >> 2);
   const uint32_t stx = (tx + 1) >> 1, sty = (ty + 3) >> 2;
   const uint32_t per_cam = stx * sty * 8u;
+  const uint32_t nsub = 32u / a.lanes, tile = sub / nsub;
   cam = (int)(tile / per_cam);
   const uint32_t r = tile % per_cam, st = r >> 3, w = r & 7u;
-  const int lane = threadIdx.x & 31;
-  x = (int)(((st % stx) * 2u + (w & 1u)) * 8u) + (lane & 7);
-  y = (int)(((st / stx) * 4u + (w >> 1)) * 4u) + (lane >> 3);
+  const uint32_t lane = threadIdx.x & 31u, p = (sub % nsub) * a.lanes + lane;
+  if (lane >= a.lanes) return false;
+  x = (int)(((st % stx) * 2u + (w & 1u)) * 8u + ((p & 3u) | ((p >> 2) & 4u)));
+  y = (int)(((st / stx) * 4u + (w >> 1)) * 4u + ((p >> 2) & 3u));
   return cam < a.ncams && x < a.width && y < a.height;
 }
 
@@ -67,13 +71,14 @@ __device__ __forceinline__ uint32_t rgba8_of(float r, float g, float b, float al
 template <int P, int kMinBlocks, bool kSkip>
 __global__ void __launch_bounds__(kMarchThreads, 2 * kMinBlocks) volume_forward_kernel(VolumeArgs a) {
   // the launch's tiles (a range of them for a frame split across GPUs)
-  const uint32_t n_tiles = a.tile_end ? a.tile_end : tile_ids(a);
+  const uint32_t nsub = 32u / a.lanes;
+  const uint32_t n_subs = (a.tile_end ? a.tile_end : tile_ids(a)) * nsub;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   bool bad = false;
-  for (uint32_t tile = a.tile_begin + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-       tile < n_tiles; tile += warps) {
+  for (uint32_t sub = a.tile_begin * nsub + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+       sub < n_subs; sub += warps) {
     int cam, x, y;
-    if (!ray_of_thread(a, tile, cam, x, y)) continue;
+    if (!ray_of_thread(a, sub, cam, x, y)) continue;
     float o[3], d[3];
     pixel_ray(a.cam[cam], x, y, o, d);
     NoVis nv;
@@ -163,13 +168,13 @@ struct GradVis {
 template <int P, int kMinBlocks>
 // grid nodes are read through L1 (see prefer_l1)
 __global__ void __launch_bounds__(kMarchThreads, 2 * kMinBlocks) volume_backward_kernel(VolumeArgs a) {
-  const uint32_t n_tiles = tile_ids(a);
+  const uint32_t n_subs = tile_ids(a) * (32u / a.lanes);
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   bool bad = false;
-  for (uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile < n_tiles;
-       tile += warps) {
+  for (uint32_t sub = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); sub < n_subs;
+       sub += warps) {
     int cam, x, y;
-    if (!ray_of_thread(a, tile, cam, x, y)) continue;
+    if (!ray_of_thread(a, sub, cam, x, y)) continue;
     const size_t off = ((size_t)cam * a.height + (size_t)y) * a.width + (size_t)x;
     const float4 g4 = reinterpret_cast<const float4*>(a.grad_rgba)[off];
     if (g4.x == 0.f && g4.y == 0.f && g4.z == 0.f && g4.w == 0.f) continue;
@@ -311,11 +316,32 @@ uint32_t volume_tiles_per_camera(int width, int height) {
   return ((tx + 1) >> 1) * ((ty + 3) >> 2) * 8u;
 }
 
-cudaError_t launch_volume_forward(const VolumeArgs& a, cudaStream_t s) {
+// Rays a warp marches (a.lanes): 32, or 16 or 8 while the launch's rays so
+// split still fit the resident warps.  A warp runs every cell and sample that
+// any of its rays takes, so a launch too small to fill the GPU ends sooner
+// with fewer rays to a warp (4 cameras at 64x64, 128^3 volume, forward and
+// backward: 1518 us at 32 rays, 1083 at 8).  24 warps: the resident warps an
+// SM holds at the kernels' register budgets (the fp32 forward's 32 gained
+// nothing more).
+static void set_lanes(VolumeArgs& a, uint64_t tiles) {
+  const uint64_t resident = (uint64_t)device_sm_count_vol() * 24u;
+  a.lanes = 32;
+  if (a.tile_end > 1u << 29) return;  // a range's part ids stay below 2^32
+  while (a.lanes > 8u && tiles * (64u / a.lanes) <= resident) a.lanes /= 2;
+}
+
+// Blocks of a launch over `tiles` tiles.
+static uint32_t march_blocks(const VolumeArgs& a, uint32_t tiles) {
+  constexpr uint32_t kWarps = kMarchThreads / 32;
+  return (uint32_t)(((uint64_t)tiles * (32u / a.lanes) + kWarps - 1) / kWarps);
+}
+
+cudaError_t launch_volume_forward(VolumeArgs& a, cudaStream_t s) {
   const uint32_t end = a.tile_end ? a.tile_end : tile_ids(a);
   const uint32_t tiles = end > a.tile_begin ? end - a.tile_begin : 0u;
-  const uint32_t blocks = (tiles + kMarchThreads / 32 - 1) / (kMarchThreads / 32);
-  if (blocks == 0) return cudaSuccess;
+  if (tiles == 0) return cudaSuccess;
+  set_lanes(a, tiles);
+  const uint32_t blocks = march_blocks(a, tiles);
   prefer_l1();
   const bool skip = a.v.cell_mask != nullptr;
   switch (a.v.precision) {
@@ -348,10 +374,11 @@ cudaError_t launch_volume_forward(const VolumeArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_volume_backward(const VolumeArgs& a, cudaStream_t s) {
+cudaError_t launch_volume_backward(VolumeArgs& a, cudaStream_t s) {
   const uint32_t tiles = tile_ids(a);
-  const uint32_t blocks = (tiles + kMarchThreads / 32 - 1) / (kMarchThreads / 32);
-  if (blocks == 0) return cudaSuccess;
+  if (tiles == 0) return cudaSuccess;
+  set_lanes(a, tiles);
+  const uint32_t blocks = march_blocks(a, tiles);
   prefer_l1();
   // only fp32 (learnable) volumes have an adjoint
   if (a.v.precision == 1)
