@@ -510,6 +510,28 @@ yv_status yv_volume_sync_aprons(const yv_volume_device* vol, float* density,
 yv_status yv_volume_pack(const float* density, const float* albedo,
                          uint32_t npoints, float* packed, void* stream);
 
+/* The forward of one step of fitting fp32 parameters: packs density
+ * (nbricks * 729) and albedo (nbricks * 729 * 3) into `packed` (as
+ * yv_volume_pack) and renders the ncams frames of the packed pool into rgba
+ * (as yv_volume_render: the same values).  vol gives the tree, nbricks and
+ * brick_bits; its density, albedo, precision and cell_mask are not read.
+ * mask: device scratch of YV_TRAIN_MASK_WORDS(nbricks) words, free for other
+ * use once the call's work on `stream` is done. */
+#define YV_TRAIN_MASK_WORDS(nbricks) ((size_t)(nbricks) * 17u)
+yv_status yv_volume_train_forward(const yv_volume_device* vol, const float* density,
+                                  const float* albedo, const yv_camera* cams,
+                                  int32_t ncams, int32_t width, int32_t height,
+                                  const yv_march_params* mp, float* packed,
+                                  uint32_t* mask, float* rgba, void* stream);
+/* Its backward: yv_volume_backward into zeroed gradients followed by
+ * yv_volume_fold_aprons, in one call that WRITES grad_density and
+ * grad_albedo (their contents before do not matter). */
+yv_status yv_volume_train_backward(const yv_volume_device* vol, const yv_camera* cams,
+                                   int32_t ncams, int32_t width, int32_t height,
+                                   const yv_march_params* mp, const float* rgba,
+                                   const float* grad_rgba, float* grad_density,
+                                   float* grad_albedo, void* stream);
+
 /* ------------------------------------------------------------------------ */
 /* Batched persistent render (no reference code; nearest structure is the   */
 /* SPU tile loop, cell/spu/trace_spu.cpp:162-177)                           */

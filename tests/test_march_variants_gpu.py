@@ -1,5 +1,7 @@
 """Variants of the brick march against each other: warps that march 8, 16 or 32
-rays."""
+rays, and the fitting step's forward (empty cells passed over) and backward
+(gradients folded in one pass) against the plain entry points they stand for."""
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -38,3 +40,65 @@ def test_small_launches_equal_large_ones(yoxel_mod, size):
         assert torch.equal(one[0], many[k])
     if w * h >= 4096:  # (a frame of few pixels has its corner rays only)
         assert float(many.abs().sum()) > 0
+
+
+@pytest.mark.parametrize("kind", ["sparse", "mixed", "dense"])
+@pytest.mark.parametrize("levels", [1, 2])
+def test_fitting_forward_equals_plain_march(yoxel_mod, kind, levels):
+    import torch
+    tv = volume(yoxel_mod, levels, kind)
+    cams = yoxel_mod.sphere_cameras(3)
+    got = yoxel_mod.volume_march(tv["density"], tv["albedo"], tv, cams, 93, 61, 1.5, 0.5)
+    packed = yoxel_mod.pack_volume(tv["density"], tv["albedo"])
+    ref = yoxel_mod.render_volume(yoxel_mod.torch_desc(tv, packed=packed), cams, 93, 61, 1.5, 0.5)
+    assert torch.equal(got, ref)
+    assert float(ref[..., 3].max()) > 0.5
+
+
+def test_not_finite_values_reach_the_frame(yoxel_mod):
+    """NaN and infinity in the parameters show where the plain march shows
+    them, also in cells whose densities are all zero."""
+    import torch
+    tv = volume(yoxel_mod, 1, "sparse")
+    den, alb = tv["density"].clone(), tv["albedo"].clone()
+    empty = (den == 0).nonzero()
+    for i, v in enumerate((float("nan"), float("inf"), float("-inf"))):
+        b, p = empty[(i + 1) * len(empty) // 5].tolist()
+        alb[b, p, i] = v
+    b, p = (den > 0).nonzero()[7].tolist()
+    den[b, p] = float("nan")
+    cams = yoxel_mod.sphere_cameras(6)
+    got = yoxel_mod.volume_march(den, alb, tv, cams, 64, 64)
+    packed = yoxel_mod.pack_volume(den, alb)
+    ref = yoxel_mod.render_volume(yoxel_mod.torch_desc(tv, packed=packed), cams, 64, 64)
+    assert bool(ref.isnan().any())
+    assert torch.equal(got.nan_to_num(nan=-7.0), ref.nan_to_num(nan=-7.0))
+
+
+@pytest.mark.parametrize("kind", ["sparse", "dense"])
+@pytest.mark.parametrize("size", [(16, 16), (250, 246)])
+def test_fitting_backward_equals_backward_and_fold(yoxel_mod, kind, size):
+    import torch
+    tv = volume(yoxel_mod, 1, kind)
+    den = tv["density"].clone().requires_grad_(True)
+    alb = tv["albedo"].clone().requires_grad_(True)
+    cams = yoxel_mod.sphere_cameras(2)
+    w, h = size
+    rgba = yoxel_mod.volume_march(den, alb, tv, cams, w, h)
+    g = torch.from_numpy(np.random.default_rng(3).standard_normal(rgba.shape).astype(np.float32))
+    g = g.cuda()
+    gd, ga = torch.autograd.grad(rgba, (den, alb), g)
+    packed = yoxel_mod.pack_volume(den.detach(), alb.detach())
+    rd, ra = torch.zeros_like(gd), torch.zeros_like(ga)
+    yoxel_mod.volume_backward(yoxel_mod.torch_desc(tv, packed=packed), cams, w, h, rgba.detach(),
+                              g, rd, ra)
+    # FP32 sums of the same terms in another order (atomics): up to some
+    # thousand per point, sqrt(4096) 2^-24 = 4e-6
+    for a, b in ((gd, rd), (ga, ra)):
+        assert float((a - b).norm() / b.norm()) < 4e-6
+    # far-side copies equal their owners, 0 where there is none
+    up = tv["nbr_up"].cpu().numpy()
+    v = gd.cpu().numpy().reshape(-1, 9, 9, 9)
+    for b in range(len(v)):
+        own = v[up[b, 0], :8, :8, 0] if up[b, 0] >= 0 else 0.0
+        assert np.array_equal(v[b, :8, :8, 8], np.broadcast_to(own, (8, 8)))

@@ -440,23 +440,24 @@ yv_status yv_volume_render_rgba8(const yv_volume_device* vol, const yv_camera* c
   return YV_OK;
 }
 
-yv_status yv_volume_backward(const yv_volume_device* vol, const yv_camera* cams, int32_t ncams,
-                             int32_t width, int32_t height, const yv_march_params* mp,
-                             const float* rgba, const float* grad_rgba, float* grad_density,
-                             float* grad_albedo, void* stream) {
+}  // extern "C"
+
+// The adjoint of the ncams frames into a packed (albedo rgb, density) float4
+// per lattice point - one 16-byte atomic per corner - taken from the
+// stream-ordered pool, then `finish(args, packed)` on the same stream.
+template <class Finish>
+static yv_status run_backward(const yv_volume_device* vol, const yv_camera* cams, int32_t ncams,
+                              int32_t width, int32_t height, const yv_march_params* mp,
+                              const float* rgba, const float* grad_rgba, cudaStream_t s,
+                              Finish finish) {
   VolumeArgs* a = new (std::nothrow) VolumeArgs;
   if (!a) return YV_ERR_OUT_OF_MEMORY;
   if (!fill_args(vol, mp, width, height, a) || !cams_ok(cams, ncams) || !rgba || !grad_rgba ||
-      !grad_density || !grad_albedo ||
       (vol->precision != YV_PRECISION_F32 && vol->precision != YV_PRECISION_F32_PACKED)) {
     delete a;
     return YV_ERR_INVALID_ARG;
   }
   const size_t px = (size_t)width * (size_t)height;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // Gradients accumulate in a packed (albedo rgb, density) float4 per
-  // lattice point - one 16-byte atomic per corner - taken from the
-  // stream-ordered pool and added into the caller's tensors at the end.
   const size_t npts = (size_t)vol->nbricks * 729u;
   float4* packed = nullptr;
   cudaError_t e = cudaSuccess;
@@ -469,19 +470,79 @@ yv_status yv_volume_backward(const yv_volume_device* vol, const yv_camera* cams,
     set_cams(a, cams + c0, n);
     a->rgba_fwd = rgba + (size_t)c0 * px * 4;
     a->grad_rgba = grad_rgba + (size_t)c0 * px * 4;
-    a->grad_density = grad_density;
-    a->grad_albedo = grad_albedo;
     a->grad_packed = packed;
     e = launch_volume_backward(*a, s);
   }
-  if (e == cudaSuccess && npts)
-    e = launch_unpack_grads(packed, (uint32_t)npts, grad_density, grad_albedo, s);
+  if (e == cudaSuccess && npts) e = finish(*a, packed);
   if (packed) {
     cudaError_t ef = scratch_free(packed, s);
     if (e == cudaSuccess) e = ef;
   }
   delete a;
   return e == cudaSuccess ? YV_OK : fail(e, "volume backward");
+}
+
+extern "C" {
+
+yv_status yv_volume_backward(const yv_volume_device* vol, const yv_camera* cams, int32_t ncams,
+                             int32_t width, int32_t height, const yv_march_params* mp,
+                             const float* rgba, const float* grad_rgba, float* grad_density,
+                             float* grad_albedo, void* stream) {
+  if (!grad_density || !grad_albedo) return YV_ERR_INVALID_ARG;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  return run_backward(vol, cams, ncams, width, height, mp, rgba, grad_rgba, s,
+                      [&](const VolumeArgs& a, const float4* packed) {
+                        return launch_unpack_grads(packed, a.v.nbricks * 729u, grad_density,
+                                                   grad_albedo, s);
+                      });
+}
+
+yv_status yv_volume_train_forward(const yv_volume_device* vol, const float* density,
+                                  const float* albedo, const yv_camera* cams, int32_t ncams,
+                                  int32_t width, int32_t height, const yv_march_params* mp,
+                                  float* packed, uint32_t* mask, float* rgba, void* stream) {
+  if (!vol || (vol->nbricks && (!density || !albedo || !packed || !mask ||
+                                (reinterpret_cast<uintptr_t>(packed) & 15u))))
+    return YV_ERR_INVALID_ARG;
+  yv_volume_device d = *vol;
+  d.density = nullptr;
+  d.albedo = packed;
+  d.precision = YV_PRECISION_F32_PACKED;
+  d.cell_mask = d.nbricks ? mask : nullptr;
+  VolumeArgs* a = new (std::nothrow) VolumeArgs;
+  if (!a) return YV_ERR_OUT_OF_MEMORY;
+  if (!fill_args(&d, mp, width, height, a) || !cams_ok(cams, ncams) || !rgba) {
+    delete a;
+    return YV_ERR_INVALID_ARG;
+  }
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  uint32_t* marked = d.nbricks ? mask + (size_t)d.nbricks * 16u : nullptr;
+  a->marked = marked;
+  const size_t px = (size_t)width * (size_t)height;
+  cudaError_t e = launch_pack_train(density, albedo, d.nbricks, reinterpret_cast<float4*>(packed),
+                                    mask, marked, s);
+  for (int c0 = 0; c0 < ncams && e == cudaSuccess; c0 += kMaxVolumeCams) {
+    const int n = ncams - c0 < kMaxVolumeCams ? ncams - c0 : kMaxVolumeCams;
+    set_cams(a, cams + c0, n);
+    a->rgba = rgba + (size_t)c0 * px * 4;
+    e = launch_volume_forward(*a, s);
+  }
+  delete a;
+  return e == cudaSuccess ? YV_OK : fail(e, "volume forward launch");
+}
+
+yv_status yv_volume_train_backward(const yv_volume_device* vol, const yv_camera* cams,
+                                   int32_t ncams, int32_t width, int32_t height,
+                                   const yv_march_params* mp, const float* rgba,
+                                   const float* grad_rgba, float* grad_density,
+                                   float* grad_albedo, void* stream) {
+  if (!vol || !vol->nbr_up || !vol->nbr_dn || !grad_density || !grad_albedo)
+    return YV_ERR_INVALID_ARG;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  return run_backward(vol, cams, ncams, width, height, mp, rgba, grad_rgba, s,
+                      [&](const VolumeArgs& a, const float4* packed) {
+                        return launch_fold_packed(a, packed, grad_density, grad_albedo, s);
+                      });
 }
 
 yv_status yv_volume_fold_aprons(const yv_volume_device* vol, float* grad_density,

@@ -91,10 +91,10 @@ __global__ void __launch_bounds__(256, kMinBlocks) batch_kernel(BatchLaunch b) {
           NoVis nv;
           RayOut r;
           switch (kP >= 0 ? kP : it.vol.precision) {
-            case 0: march<0>(it.vol, o, d, nv, r); break;
-            case 1: march<1>(it.vol, o, d, nv, r); break;
-            case 2: march<2>(it.vol, o, d, nv, r); break;
-            default: march<3>(it.vol, o, d, nv, r); break;
+            case 0: march<0>(it.vol, o, d, nv, r, it.vol.cell_mask != nullptr); break;
+            case 1: march<1>(it.vol, o, d, nv, r, it.vol.cell_mask != nullptr); break;
+            case 2: march<2>(it.vol, o, d, nv, r, it.vol.cell_mask != nullptr); break;
+            default: march<3>(it.vol, o, d, nv, r, it.vol.cell_mask != nullptr); break;
           }
           if (r.bad) err |= YV_DEV_ERR_POOL;
           reinterpret_cast<float4*>(it.frgba)[off] = make_float4(r.c[0], r.c[1], r.c[2], r.a);

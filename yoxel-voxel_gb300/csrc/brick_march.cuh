@@ -347,10 +347,10 @@ __device__ __forceinline__ void march_enter(const VolumeView& a, const float* o,
 // kColor = false (the adjoint's replay): the composited colour is not
 // accumulated (the visitor tracks what it needs; r.c stays 0).
 // kSkip: the forward passes over the samples of cells the pool's
-// cell_mask marks empty (compiled out for pools without one).
+// cell_mask marks empty where `masked` (compiled out for pools without one).
 template <int P, class Vis, bool kColor = true, bool kSkip = kColor>
 __device__ __forceinline__ void march(const VolumeView& a, const float* o, const float* d,
-                                      Vis& vis, RayOut& r) {
+                                      Vis& vis, RayOut& r, bool masked = false) {
   r.c[0] = r.c[1] = r.c[2] = 0.f;
   r.a = 0.f;
   r.samples = 0;
@@ -376,7 +376,7 @@ __device__ __forceinline__ void march(const VolumeView& a, const float* o, const
           sample_coord(m.t, m.D[i], m.Lh[i], m.Ll[i], lc[i], le[i]);
           kb[i] = cell_of(lc[i]);
         }
-        if (kColor && kSkip && a.cell_mask && !cell_marked(a, b, kb)) {
+        if (kColor && kSkip && masked && !cell_marked(a, b, kb)) {
           // a cell whose 8 corners are all zero has sigma = 0, alpha = 0:
           // the sample adds exactly nothing (C, A unchanged), so the
           // forward passes over it; the replay of the adjoint, whose

@@ -24,6 +24,7 @@
 #include <string>
 #include <vector>
 
+#include "brick_mask.cuh"
 #include "dev_scan.cuh"
 #include "yv_internal.h"
 #include "yv_kernels.h"
@@ -311,13 +312,6 @@ __device__ __forceinline__ uint16_t f16_saturating(float f) {
 // trilinear cell (x, y, z) has a non-zero stored density corner), from a
 // 729-bit non-zero map of the brick's lattice the warp gathers by ballots
 // while it packs (blocks of 256 threads).
-__device__ __forceinline__ uint32_t lattice_row9(const uint32_t* bits, int off) {
-  const int w = off >> 5, sh = off & 31;
-  uint32_t v = bits[w] >> sh;
-  if (sh > 23) v |= bits[w + 1] << (32 - sh);
-  return v & 0x1FFu;
-}
-
 // bits (device pools, optional, zeroed before): the brick bitmap, bit
 // (ci & 31) of word ci >> 5 set for the cell ci = (cz nb + cy) nb + cx of
 // every brick.
@@ -409,20 +403,7 @@ __global__ void pack_bricks_kernel(Lattice g, const uint64_t* cells, uint32_t nb
     if (mask) {
       if (lane == 0) nz[23] = 0u;  // beyond the 729 points
       __syncwarp();
-      if (lane < 16u) {
-        const int z = (int)(lane >> 1), y0 = (int)(lane & 1u) * 4;
-        uint32_t word = 0;
-        for (int yy = 0; yy < 4; ++yy) {
-          uint32_t rows = 0;
-          for (int dz = 0; dz < 2; ++dz)
-            for (int dy = 0; dy < 2; ++dy) {
-              const uint32_t r9 = lattice_row9(nz, (z + dz) * 81 + (y0 + yy + dy) * 9);
-              rows |= r9 | (r9 >> 1);  // cell x holds point x or x + 1
-            }
-          word |= (rows & 0xFFu) << (8 * yy);
-        }
-        mask[(size_t)b * 16u + lane] = word;
-      }
+      if (lane < 16u) mask[(size_t)b * 16u + lane] = cell_mask_word(nz, lane);
       __syncwarp();
     }
   }

@@ -55,14 +55,15 @@ struct VolumeArgs {
   uint32_t* bricks_entered;
   const float* rgba_fwd;  // backward: forward output
   const float* grad_rgba; // backward: dL/d rgba
-  float* grad_density;    // backward outputs (pool layout)
-  float* grad_albedo;
-  float4* grad_packed;    // backward scratch: (albedo rgb, density) per lattice point
+  float4* grad_packed;    // backward output: (albedo rgb, density) per lattice point
   uint32_t* status;       // optional device status word
   // forward only: warp tiles [tile_begin, tile_end) of the launch (march
   // order, see tile_ids); tile_end = 0: all of them
   uint32_t tile_begin, tile_end;
   uint32_t lanes;  // rays a warp marches; set by the launchers
+  // forward with a cell_mask: marked cells of each brick, by which the kernel
+  // decides whether testing the mask pays; null = it does
+  const uint32_t* marked;
 };
 
 cudaError_t launch_volume_forward(VolumeArgs& a, cudaStream_t s);
@@ -73,6 +74,15 @@ cudaError_t launch_volume_backward(VolumeArgs& a, cudaStream_t s);
 // packed[i] = (albedo rgb, density) of n lattice points (fp32 layouts).
 cudaError_t launch_pack_f32(const float* density, const float* albedo, uint32_t n,
                             float4* packed, cudaStream_t s);
+// The same for the lattices of nbricks bricks, with the cell occupancy mask of
+// the packed pool (16 words per brick) and its marked cells per brick.
+cudaError_t launch_pack_train(const float* density, const float* albedo, uint32_t nbricks,
+                              float4* packed, uint32_t* mask, uint32_t* marked, cudaStream_t s);
+// grad_density / grad_albedo = the packed gradients of a.v's pool, every copy
+// of a lattice point holding the sum over its copies (0 where its owner brick
+// is absent).
+cudaError_t launch_fold_packed(const VolumeArgs& a, const float4* packed, float* grad_density,
+                               float* grad_albedo, cudaStream_t s);
 // grad_density += packed.w, grad_albedo += packed.xyz (n lattice points).
 cudaError_t launch_unpack_grads(const float4* packed, uint32_t n, float* grad_density,
                                 float* grad_albedo, cudaStream_t s);

@@ -193,6 +193,11 @@ _SIGS = {
     "yv_volume_fold_aprons": (S, [C.POINTER(VolumeDevice), P, P, P]),
     "yv_volume_sync_aprons": (S, [C.POINTER(VolumeDevice), P, P, P]),
     "yv_volume_pack": (S, [P, P, C.c_uint32, P, P]),
+    "yv_volume_train_forward": (S, [C.POINTER(VolumeDevice), P, P, C.POINTER(Camera), C.c_int32,
+                                    C.c_int32, C.c_int32, C.POINTER(MarchParams), P, P, P, P]),
+    "yv_volume_train_backward": (S, [C.POINTER(VolumeDevice), C.POINTER(Camera), C.c_int32,
+                                     C.c_int32, C.c_int32, C.POINTER(MarchParams), P, P, P, P,
+                                     P]),
     "yv_batch_create": (S, [C.POINTER(P)]),
     "yv_batch_destroy": (None, [P]),
     "yv_batch_clear": (S, [P]),

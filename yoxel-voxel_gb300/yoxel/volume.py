@@ -367,16 +367,25 @@ def _make_function():
         """rgba = march(density, albedo); backward re-marches each ray.
 
         The parameters are packed once per forward into the float4
-        (r, g, b, density) pool, which both passes read."""
+        (r, g, b, density) pool, which both passes read, together with the
+        cell occupancy mask that lets the forward pass over empty cells."""
 
         @staticmethod
         def forward(ctx, density, albedo, tv, cams, width, height, alpha_scale, step_vox):
             density = density.contiguous()
             albedo = albedo.contiguous()
-            packed = pack_volume(density, albedo)
+            nb = density.shape[0]
+            packed = torch.empty((nb, 729, 4), dtype=torch.float32, device=density.device)
+            mask = torch.empty(nb * 17, dtype=torch.int32, device=density.device)
             desc = torch_desc(tv, packed=packed)
             ca = cams if isinstance(cams, C.Array) else cameras(cams)
-            rgba = render_volume(desc, ca, width, height, alpha_scale, step_vox)
+            rgba = torch.empty((len(ca), height, width, 4), dtype=torch.float32, device="cuda")
+            mp = L.MarchParams(float(alpha_scale), float(step_vox))
+            L.check(L.lib.yv_volume_train_forward(
+                C.byref(desc), C.c_void_p(density.data_ptr()), C.c_void_p(albedo.data_ptr()), ca,
+                len(ca), width, height, C.byref(mp), C.c_void_p(packed.data_ptr()),
+                C.c_void_p(mask.data_ptr()), C.c_void_p(rgba.data_ptr()), _stream(None)),
+                "yv_volume_train_forward")
             ctx.save_for_backward(packed, rgba)
             ctx.meta = (tv, ca, width, height, alpha_scale, step_vox, density.shape, albedo.shape)
             return rgba
@@ -385,11 +394,16 @@ def _make_function():
         def backward(ctx, grad_rgba):
             packed, rgba = ctx.saved_tensors
             tv, ca, width, height, alpha_scale, step_vox, dshape, ashape = ctx.meta
-            gd = torch.zeros(dshape, dtype=torch.float32, device=packed.device)
-            ga = torch.zeros(ashape, dtype=torch.float32, device=packed.device)
+            gd = torch.empty(dshape, dtype=torch.float32, device=packed.device)
+            ga = torch.empty(ashape, dtype=torch.float32, device=packed.device)
             desc = torch_desc(tv, packed=packed)
-            volume_backward(desc, ca, width, height, rgba, grad_rgba.contiguous(), gd, ga,
-                            alpha_scale, step_vox)
+            grad_rgba = grad_rgba.contiguous()
+            mp = L.MarchParams(float(alpha_scale), float(step_vox))
+            L.check(L.lib.yv_volume_train_backward(
+                C.byref(desc), ca, len(ca), width, height, C.byref(mp),
+                C.c_void_p(rgba.data_ptr()), C.c_void_p(grad_rgba.data_ptr()),
+                C.c_void_p(gd.data_ptr()), C.c_void_p(ga.data_ptr()), _stream(None)),
+                "yv_volume_train_backward")
             return gd, ga, None, None, None, None, None, None
 
     return VolumeMarch
