@@ -102,3 +102,16 @@ def test_fitting_backward_equals_backward_and_fold(yoxel_mod, kind, size):
     for b in range(len(v)):
         own = v[up[b, 0], :8, :8, 0] if up[b, 0] >= 0 else 0.0
         assert np.array_equal(v[b, :8, :8, 8], np.broadcast_to(own, (8, 8)))
+
+
+@pytest.mark.parametrize("precision", [0, 1, 2, 3])
+def test_register_budgets_agree(yoxel_mod, precision):
+    """A launch whose warps all fit at the small register budget, and one that
+    does not, of every lattice format."""
+    import torch
+    gv = yoxel_mod.BrickVolume.noise(1, 0.4, 1.4, 8).upload(precision)
+    cams = yoxel_mod.sphere_cameras(50)
+    many = yoxel_mod.render_volume(gv.desc(), cams, 67, 43)
+    for k in (0, 31):
+        assert torch.equal(yoxel_mod.render_volume(gv.desc(), [cams[k]], 67, 43)[0], many[k])
+    assert float(many[..., 3].max()) > 0.1

@@ -5,6 +5,8 @@
 #include "brick_march.cuh"
 #include "brick_mask.cuh"
 
+#include <atomic>
+
 namespace yv {
 namespace {
 
@@ -13,18 +15,16 @@ namespace {
 // work: 64-camera training step 10.04 ms at 256 threads, 9.66 at 128, 9.79 at
 // 64; 1024^2 frame of a 512^3 volume 740 / 704 / 719 us.
 constexpr int kMarchThreads = 128;
-// Register budget of the adjoint (resident warps per SM / 8): its 16
-// per-lane gradient accumulators live in registers (a shared-memory copy
-// measured 1.25x slower).
-constexpr int kBackwardMinBlocks = 3;
-// Register budget of the forward march per lattice format (resident warps
-// per SM / 8): 3 for the fp16 + 8-bit colour formats (0, 3), 4 for the fp32
-// formats (1, 2).  1024^2 frame of a 512^3 volume, 8-byte format: 740 us at 3,
-// 764 at 4; 64-camera fp32 training step 10.04 ms at 4, 10.13 at 3.
-template <int P>
-struct ForwardBlocks {
-  static constexpr int value = (P == 0 || P == 3) ? 3 : 4;
-};
+// Register budgets (resident warps per SM / 8).  A launch that fills the GPU
+// runs at 3: adjoint of a 64-camera fitting step of a 128^3 volume 6.5 ms (2:
+// 6.9, 4: 6.9 with spills); forward of the fp32 formats alike at 3 and 4 there
+// and 7 % faster at 3 on a volume without empty cells; 8-byte format 1024^2
+// of a 512^3 volume 740 us at 3, 764 at 4.  A launch whose warps all fit at 2
+// is bound by the latency of its longest warp and runs there, where nothing
+// spills and more loads are in flight: 4 cameras at 64x64, forward and
+// backward, 693 -> 493 us.
+constexpr int kMinBlocks = 3;
+constexpr int kSmallMinBlocks = 2;
 
 // tile mapping: warp w of the grid -> 8x4 pixel tile of one camera image;
 // 8 consecutive tiles are a 2x4-tile (16x16-pixel) square
@@ -75,14 +75,14 @@ __device__ __forceinline__ bool mask_pays(const VolumeArgs& a) {
   return __reduce_add_sync(0xFFFFFFFFu, __ldg(a.marked + b)) < 32u * 512u * 45u / 100u;
 }
 
-// kMinBlocks: resident warps per SM / 8 the register allocation is sized for.
+// kBlocks: resident warps per SM / 8 the register allocation is sized for.
 // Bound by instruction issue.  On the 1024^2 frame of a 512^3 volume (8-byte
 // format) 876 -> 740 us from the cell found by one round-down add instead of
 // a conversion and clamps, the fraction clamped by the add's saturation, and
 // the half decoded by one conversion; 704 us with blocks of 128 threads.
 // kSkip: the pool carries a cell occupancy mask (a learnable pool does not).
-template <int P, int kMinBlocks, bool kSkip>
-__global__ void __launch_bounds__(kMarchThreads, 2 * kMinBlocks) volume_forward_kernel(VolumeArgs a) {
+template <int P, int kBlocks, bool kSkip>
+__global__ void __launch_bounds__(kMarchThreads, 2 * kBlocks) volume_forward_kernel(VolumeArgs a) {
   // the launch's tiles (a range of them for a frame split across GPUs)
   const uint32_t nsub = 32u / a.lanes;
   const uint32_t n_subs = (a.tile_end ? a.tile_end : tile_ids(a)) * nsub;
@@ -143,8 +143,7 @@ struct GradVis {
   float gout;   // g . (forward output of this ray)
   float gb;     // g . (r, g, b, A) composited before the current sample
   uint32_t base;
-  float gd[8];  // density
-  float gw[8];  // colour weight
+  f32x2 acc[8];  // (density, colour weight)
   __device__ __forceinline__ void init() {
     base = 0xFFFFFFFFu;
     gb = 0.f;
@@ -152,36 +151,33 @@ struct GradVis {
   __device__ __forceinline__ void flush() {
     if (base == 0xFFFFFFFFu) return;
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 8; ++j) {
+      float gd, gw;
+      unpack2(acc[j], gd, gw);
       atomicAdd(a->grad_packed + base + corner_offset(j),
-                make_float4(fmul(g[0], gw[j]), fmul(g[1], gw[j]), fmul(g[2], gw[j]), gd[j]));
+                make_float4(fmul(g[0], gw), fmul(g[1], gw), fmul(g[2], gw), gd));
+    }
   }
   __device__ __forceinline__ void operator()(const SampleCtx& s, float T, float w) {
     const float gc = ffma(g[2], s.col[2], ffma(g[1], s.col[1], ffma(g[0], s.col[0], g[3])));
     const float ds = sample_dsigma(a, gc, gout, gb, s, T, w);
     gb = ffma(w, gc, gb);
+    const f32x2 v = pack2(ds, w);
     if (s.base != base) {
       flush();
       base = s.base;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        gd[j] = fmul(s.w[j], ds);
-        gw[j] = fmul(s.w[j], w);
-      }
+      for (int j = 0; j < 8; ++j) acc[j] = mul2(pack2(s.w[j], s.w[j]), v);
     } else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        gd[j] = ffma(s.w[j], ds, gd[j]);
-        gw[j] = ffma(s.w[j], w, gw[j]);
-      }
+      for (int j = 0; j < 8; ++j) acc[j] = fma2(pack2(s.w[j], s.w[j]), v, acc[j]);
     }
   }
 };
 
-// kMinBlocks: register budget (resident warps per SM / 8).
-template <int P, int kMinBlocks>
-// grid nodes are read through L1 (see prefer_l1)
-__global__ void __launch_bounds__(kMarchThreads, 2 * kMinBlocks) volume_backward_kernel(VolumeArgs a) {
+// kBlocks: resident warps per SM / 8 the register allocation is sized for.
+template <int P, int kBlocks>
+__global__ void __launch_bounds__(kMarchThreads, 2 * kBlocks) volume_backward_kernel(VolumeArgs a) {
   const uint32_t n_subs = tile_ids(a) * (32u / a.lanes);
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   bool bad = false;
@@ -296,31 +292,41 @@ __global__ void fold_scatter_kernel(VolumeArgs a, int channels, float* g) {
 // 1365 -> 1434 Mrays/s and adjoint 6.65 -> 6.40 ms; 512^3 fp16 + RGB8
 // frame 875 -> 907 Mrays/s (the lowest carveout that still held the staged
 // nodes gave half of these gains).
-void prefer_l1() {
-  static bool done[64] = {false};
+template <void (*kKernel)(VolumeArgs)>
+void launch_march(const VolumeArgs& a, uint32_t blocks, cudaStream_t s) {
+  static std::atomic<bool> done[64];
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || done[dev]) return;
-  const cudaFuncAttribute k = cudaFuncAttributePreferredSharedMemoryCarveout;
-  const cudaError_t e[10] = {
-      cudaFuncSetAttribute(volume_forward_kernel<0, ForwardBlocks<0>::value, false>, k, 0),
-      cudaFuncSetAttribute(volume_forward_kernel<0, ForwardBlocks<0>::value, true>, k, 0),
-      cudaFuncSetAttribute(volume_forward_kernel<1, ForwardBlocks<1>::value, false>, k, 0),
-      cudaFuncSetAttribute(volume_forward_kernel<1, ForwardBlocks<1>::value, true>, k, 0),
-      cudaFuncSetAttribute(volume_forward_kernel<2, ForwardBlocks<2>::value, false>, k, 0),
-      cudaFuncSetAttribute(volume_forward_kernel<2, ForwardBlocks<2>::value, true>, k, 0),
-      cudaFuncSetAttribute(volume_forward_kernel<3, ForwardBlocks<3>::value, false>, k, 0),
-      cudaFuncSetAttribute(volume_forward_kernel<3, ForwardBlocks<3>::value, true>, k, 0),
-      cudaFuncSetAttribute(volume_backward_kernel<1, kBackwardMinBlocks>, k, 0),
-      cudaFuncSetAttribute(volume_backward_kernel<2, kBackwardMinBlocks>, k, 0)};
-  // a hint: a refusal keeps the default configuration and is not reported
-  // as the next launch's error
-  for (cudaError_t x : e)
-    if (x != cudaSuccess) {
+  if (dev >= 0 && dev < 64 && !done[dev].load(std::memory_order_relaxed)) {
+    // a hint: a refusal keeps the default configuration and is not reported
+    // as the launch's error
+    if (cudaFuncSetAttribute(kKernel, cudaFuncAttributePreferredSharedMemoryCarveout, 0) !=
+        cudaSuccess)
       cudaGetLastError();
-      break;
-    }
-  done[dev] = true;
+    done[dev].store(true, std::memory_order_relaxed);
+  }
+  kKernel<<<blocks, kMarchThreads, 0, s>>>(a);
+}
+
+// Whether every warp of a march is resident at the small budget.
+bool fits_small(uint32_t blocks) {
+  return blocks <= (uint32_t)device_sm_count_vol() * 2u * (uint32_t)kSmallMinBlocks;
+}
+
+template <int P, bool kSkip>
+void launch_forward(const VolumeArgs& a, uint32_t blocks, cudaStream_t s) {
+  if (fits_small(blocks))
+    launch_march<volume_forward_kernel<P, kSmallMinBlocks, kSkip>>(a, blocks, s);
+  else
+    launch_march<volume_forward_kernel<P, kMinBlocks, kSkip>>(a, blocks, s);
+}
+
+template <int P>
+void launch_backward(const VolumeArgs& a, uint32_t blocks, cudaStream_t s) {
+  if (fits_small(blocks))
+    launch_march<volume_backward_kernel<P, kSmallMinBlocks>>(a, blocks, s);
+  else
+    launch_march<volume_backward_kernel<P, kMinBlocks>>(a, blocks, s);
 }
 
 }  // namespace
@@ -356,33 +362,12 @@ cudaError_t launch_volume_forward(VolumeArgs& a, cudaStream_t s) {
   if (tiles == 0) return cudaSuccess;
   set_lanes(a, tiles);
   const uint32_t blocks = march_blocks(a, tiles);
-  prefer_l1();
   const bool skip = a.v.cell_mask != nullptr;
   switch (a.v.precision) {
-    case 0:
-      if (skip)
-        volume_forward_kernel<0, ForwardBlocks<0>::value, true><<<blocks, kMarchThreads, 0, s>>>(a);
-      else
-        volume_forward_kernel<0, ForwardBlocks<0>::value, false><<<blocks, kMarchThreads, 0, s>>>(a);
-      break;
-    case 1:
-      if (skip)
-        volume_forward_kernel<1, ForwardBlocks<1>::value, true><<<blocks, kMarchThreads, 0, s>>>(a);
-      else
-        volume_forward_kernel<1, ForwardBlocks<1>::value, false><<<blocks, kMarchThreads, 0, s>>>(a);
-      break;
-    case 2:
-      if (skip)
-        volume_forward_kernel<2, ForwardBlocks<2>::value, true><<<blocks, kMarchThreads, 0, s>>>(a);
-      else
-        volume_forward_kernel<2, ForwardBlocks<2>::value, false><<<blocks, kMarchThreads, 0, s>>>(a);
-      break;
-    case 3:
-      if (skip)
-        volume_forward_kernel<3, ForwardBlocks<3>::value, true><<<blocks, kMarchThreads, 0, s>>>(a);
-      else
-        volume_forward_kernel<3, ForwardBlocks<3>::value, false><<<blocks, kMarchThreads, 0, s>>>(a);
-      break;
+    case 0: skip ? launch_forward<0, true>(a, blocks, s) : launch_forward<0, false>(a, blocks, s); break;
+    case 1: skip ? launch_forward<1, true>(a, blocks, s) : launch_forward<1, false>(a, blocks, s); break;
+    case 2: skip ? launch_forward<2, true>(a, blocks, s) : launch_forward<2, false>(a, blocks, s); break;
+    case 3: skip ? launch_forward<3, true>(a, blocks, s) : launch_forward<3, false>(a, blocks, s); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -393,12 +378,11 @@ cudaError_t launch_volume_backward(VolumeArgs& a, cudaStream_t s) {
   if (tiles == 0) return cudaSuccess;
   set_lanes(a, tiles);
   const uint32_t blocks = march_blocks(a, tiles);
-  prefer_l1();
   // only fp32 (learnable) volumes have an adjoint
   if (a.v.precision == 1)
-    volume_backward_kernel<1, kBackwardMinBlocks><<<blocks, kMarchThreads, 0, s>>>(a);
+    launch_backward<1>(a, blocks, s);
   else if (a.v.precision == 2)
-    volume_backward_kernel<2, kBackwardMinBlocks><<<blocks, kMarchThreads, 0, s>>>(a);
+    launch_backward<2>(a, blocks, s);
   else
     return cudaErrorInvalidValue;
   return cudaGetLastError();
