@@ -11,13 +11,15 @@
 // grid node; bricks copy their 9^3 lattice values and RGB (white without an
 // rgb lattice); neighbour tables for the apron fold.
 //
-// Passes: a cell is marked from per-row cell bits (one warp per lattice row,
-// coalesced loads and ballots) ORed over its 9 x 9 rows;
-// one pass per level ORs 64 child flags; top-down, an exclusive scan of the
-// per-node counts of occupied children expands level l's breadth-first list
-// into level l+1's and gives every node its first child id (bricks are the
-// last level's children); emit passes write the grid refs, pack the bricks
-// (optionally straight into a device pool format) and fill the neighbours.
+// Passes: a cell is marked from per-row cell bits (the lattice read once) ORed
+// over its 9 x 9 rows, 64 cells to a mask per last-level node; one pass per
+// level above gathers the masks of its nodes; top-down, the prefix sums of the
+// masks' counts expand level l's breadth-first list into level l+1's, give
+// every node its first child and write its refs (bricks are the last level's
+// children); a last pass packs the bricks (optionally straight into a device
+// pool format) with their masks, bitmap and neighbours.  The passes over the
+// tree take their sizes from the device; the host reads the counts once,
+// before it sizes the pool.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -151,6 +153,32 @@ __global__ void mark_rows_flat_kernel(Lattice g, uint32_t* R) {
         if (left > 1u) v.y = __ldg(s1 + 1);
         if (left > 2u) v.z = __ldg(s1 + 2);
       }
+      if (xs + 128u <= L && 128u + 4u * f0 <= nfl) {
+        // all 128 points in row ra (uniform): the lane's 4 points shifted to
+        // their place among the 8 of their cell; bit 0 is also the previous
+        // cell's apron, bit 8 the first point of the next cell and this
+        // one's apron
+        const uint32_t q = (xs & 7u) + 4u * lane;
+        const uint32_t nib = (v.x != 0.f ? 1u : 0u) | (v.y != 0.f ? 2u : 0u) |
+                             (v.z != 0.f ? 4u : 0u) | (v.w != 0.f ? 8u : 0u);
+        const uint32_t p = nib << (q & 7u);
+        const uint32_t bits = (p & 1u) | ((p & 0x1FFu) ? 2u : 0u) | ((p >> 8) ? 4u : 0u);
+        // window bit 0: the cell before the warp's first
+        const uint32_t win = __reduce_or_sync(0xFFFFFFFFu, bits << (q >> 3));
+        if (lane == 0 && win) {
+          const uint32_t c = xs >> 3;
+          const uint64_t sft = c ? (uint64_t)win << ((c - 1u) & 31u) : (uint64_t)(win >> 1);
+          const uint32_t w = c ? (c - 1u) >> 5 : 0u;
+          if (w < NW) acc[ra][w] |= (uint32_t)sft;
+          if (w + 1 < NW) acc[ra][w + 1] |= (uint32_t)(sft >> 32);
+        }
+        xs += 128u;
+        if (xs >= L) {
+          xs -= L;
+          ++ra;
+        }
+        continue;
+      }
       // the warp's 128 points: rows ra (first point) .. ra + 1
       const int c_lo = (int)(xs >> 3) - 1;  // window: cells c_lo .. c_lo + 31
       const uint32_t rb = ra + 1;           // cells -1..30 of the next row
@@ -205,92 +233,160 @@ __global__ void mark_rows_flat_kernel(Lattice g, uint32_t* R) {
 }
 
 // Mark, pass 2: a cell is occupied when its bit is set in any of the 9 x 9
-// rows y in [8 cy, 8 cy + 8], z in [8 cz, 8 cz + 8].  One thread per row word
-// and (cy, cz); count = occupied cells, one atomic per warp.
-__global__ void mark_cells_from_rows_kernel(Lattice g, const uint32_t* R, uint8_t* occ,
-                                            uint32_t* count) {
+// rows y in [8 cy, 8 cy + 8], z in [8 cz, 8 cz + 8].  One warp per row word and
+// 4x4 square of (cy, cz): lane j and j + 16 OR the lower and upper rows of
+// square cell j, then the nibbles of the 16 lanes make the 64-cell mask (bit
+// x | y<<2 | z<<4) of each last-level node of the word.
+// counts[0] += nodes with a cell, counts[1] += cells.
+__global__ void __launch_bounds__(256) mark_nodes_kernel(Lattice g, const uint32_t* R,
+                                                         uint64_t* mask, uint32_t* node_count,
+                                                         uint32_t* cell_count) {
+  const uint32_t lane = threadIdx.x & 31u;
   const uint32_t NW = g.nb >= 32 ? (uint32_t)g.nb / 32u : 1u;
-  const int nbs = __ffs(g.nb) - 1;
-  const uint64_t total = (uint64_t)NW * g.nb * g.nb;
-  uint32_t my = 0;
-  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
-       t += (uint64_t)gridDim.x * blockDim.x) {
-    const int wsh = __ffs(NW) - 1;  // NW is a power of two
-    const uint32_t w = (uint32_t)(t & (NW - 1u));
-    const uint64_t yz = t >> wsh;
-    const uint32_t cy = (uint32_t)(yz & (uint64_t)(g.nb - 1)), cz = (uint32_t)(yz >> nbs);
-    uint32_t acc = 0;
-    for (int dz = 0; dz < 9; ++dz)
-      for (int dy = 0; dy < 9; ++dy)
-        acc |= R[(((uint64_t)(8 * cz + dz)) * g.L + (8 * cy + dy)) * NW + w];
-    const int nbits = g.nb >= 32 ? 32 : g.nb;
-    for (int b = 0; b < nbits; ++b)
-      occ[((uint64_t)cz << (2 * nbs)) + ((uint64_t)cy << nbs) + 32u * w + (uint32_t)b] =
-          (uint8_t)((acc >> b) & 1u);
-    my += (uint32_t)__popc(nbits == 32 ? acc : acc & ((1u << nbits) - 1u));
+  const uint32_t n = (uint32_t)g.nb / 4u;  // nodes per axis
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (warp >= NW * n * n) return;
+  const uint32_t w = warp % NW, gy = (warp / NW) % n, gz = warp / (NW * n);
+  const uint32_t y = lane & 3u, z = (lane >> 2) & 3u;
+  const uint64_t cy = 4u * gy + y, cz = 4u * gz + z;
+  const int z0 = lane < 16u ? 0 : 5, z1 = lane < 16u ? 5 : 9;
+  uint32_t acc = 0;
+  for (int dz = z0; dz < z1; ++dz) {
+    const uint32_t* p = R + ((8u * cz + (uint64_t)dz) * g.L + 8u * cy) * NW + w;
+#pragma unroll
+    for (int dy = 0; dy < 9; ++dy) acc |= __ldg(p + (uint32_t)dy * NW);
   }
-  my = __reduce_add_sync(0xFFFFFFFFu, my);
-  if ((threadIdx.x & 31u) == 0 && my) atomicAdd(count, my);
+  acc |= __shfl_xor_sync(0xFFFFFFFFu, acc, 16);
+  const uint32_t nn = n < 8u ? n : 8u;
+  uint32_t lo = 0, hi = 0;  // lane k: the mask of node k of the word
+  for (uint32_t k = 0; k < nn; ++k) {
+    const uint32_t nib = ((acc >> (4u * k)) & 15u) << (4u * y + 16u * (z & 1u));
+    const uint32_t l = __reduce_or_sync(0xFFFFFFFFu, z < 2u ? nib : 0u);
+    const uint32_t h = __reduce_or_sync(0xFFFFFFFFu, z < 2u ? 0u : nib);
+    if (lane == k) {
+      lo = l;
+      hi = h;
+    }
+  }
+  if (lane < nn)
+    mask[((uint64_t)gz * n + gy) * n + 8u * w + lane] = (uint64_t)lo | ((uint64_t)hi << 32);
+  const uint32_t cells = __reduce_add_sync(0xFFFFFFFFu, __popc(lo) + __popc(hi));
+  const uint32_t nodes = __popc(__ballot_sync(0xFFFFFFFFu, (lo | hi) != 0u));
+  if (lane == 0 && cells) {
+    atomicAdd(cell_count, cells);
+    atomicAdd(node_count, nodes);
+  }
 }
 
 // Index of child c (x | y<<2 | z<<4) of node p of a level with n = 2^s
 // nodes per axis, in the level below (4n per axis).
-__device__ __forceinline__ uint64_t child64(uint64_t p, uint32_t n, int c) {
+__device__ __forceinline__ uint32_t child64(uint32_t p, uint32_t n, uint32_t c) {
   const int s = __ffs(n) - 1;
-  const uint64_t x = p & (n - 1u), y = (p >> s) & (n - 1u), z = p >> (2 * s);
-  return (4 * x + (c & 3)) + ((4 * y + ((c >> 2) & 3)) << (s + 2)) +
+  const uint32_t x = p & (n - 1u), y = (p >> s) & (n - 1u), z = p >> (2 * s);
+  return (4 * x + (c & 3u)) + ((4 * y + ((c >> 2) & 3u)) << (s + 2)) +
          ((4 * z + (c >> 4)) << (2 * s + 4));
 }
 
-// Level l (n per axis) from level l+1 (4n per axis): OR of 64 children.
-// count: occupied nodes of the level, one atomic per warp.
-__global__ void fold64_kernel(const uint8_t* child, uint32_t n, uint8_t* out, uint32_t* count) {
-  const uint64_t total = (uint64_t)n * n * n;
-  uint32_t my = 0;
-  for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < total;
-       p += (uint64_t)gridDim.x * blockDim.x) {
-    uint8_t a = 0;
-    for (int c = 0; c < 64 && !a; ++c) a = child[child64(p, n, c)];
-    out[p] = a;
-    my += a;
-  }
-  my = __reduce_add_sync(0xFFFFFFFFu, my);
-  if ((threadIdx.x & 31u) == 0 && my) atomicAdd(count, my);
-}
-
-__global__ void count64_kernel(const uint64_t* list, uint32_t m, const uint8_t* child_any,
-                               uint32_t n, uint32_t* counts) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    uint32_t k = 0;
-    for (int c = 0; c < 64; ++c) k += child_any[child64(list[i], n, c)] ? 1u : 0u;
-    counts[i] = k;
+// Masks of level l (n per axis) from level l+1's (4n per axis), a warp per
+// node; count += nodes with a child.
+__global__ void __launch_bounds__(256) fold_masks_kernel(const uint64_t* child, uint32_t n,
+                                                         uint64_t* mask, uint32_t* count) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (p >= n * n * n) return;
+  const uint32_t lo = __ballot_sync(0xFFFFFFFFu, child[child64(p, n, lane)] != 0ull);
+  const uint32_t hi = __ballot_sync(0xFFFFFFFFu, child[child64(p, n, lane + 32u)] != 0ull);
+  if (lane == 0) {
+    mask[p] = (uint64_t)lo | ((uint64_t)hi << 32);
+    if (lo | hi) atomicAdd(count, 1u);
   }
 }
 
-__global__ void expand64_kernel(const uint64_t* list, uint32_t m, const uint8_t* child_any,
-                                uint32_t n, const uint32_t* offsets, uint64_t* next) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    uint32_t o = offsets[i];
-    for (int c = 0; c < 64; ++c) {
-      const uint64_t q = child64(list[i], n, c);
-      if (child_any[q]) next[o++] = q;
-    }
-  }
+// Nodes of level l's breadth-first list per block of the two kernels below.
+constexpr uint32_t kListChunk = 256;
+
+// counts: occupied nodes of each level ([0] unused: the root is always
+// there).  Length of level l's list.
+__device__ __forceinline__ uint32_t list_len(const uint32_t* counts, int l) {
+  return l == 0 ? 1u : counts[l];
 }
 
-// Grid refs of one level: occupied children are grid nodes (child_base +
-// rank) or, at the last level, bricks (0x40000000 | rank).
-__global__ void emit_grids_kernel(const uint64_t* list, uint32_t m, const uint8_t* child_any,
-                                  uint32_t n, const uint32_t* offsets, uint32_t node_base,
-                                  uint32_t child_base, bool bricks, uint32_t* grids) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    uint32_t next = offsets[i];
-    uint32_t* g = grids + (size_t)(node_base + i) * 64;
-    for (int c = 0; c < 64; ++c) {
+// Children per chunk of level l's list.
+__global__ void __launch_bounds__(kListChunk) child_sums_kernel(const uint32_t* counts, int l,
+                                                                const uint32_t* list,
+                                                                const uint64_t* mask,
+                                                                uint32_t* sums) {
+  const uint32_t m = list_len(counts, l), i = blockIdx.x * kListChunk + threadIdx.x;
+  if (blockIdx.x * kListChunk >= m) return;
+  __shared__ uint32_t tot;
+  if (threadIdx.x == 0) tot = 0;
+  __syncthreads();
+  uint32_t c = i < m ? (uint32_t)__popcll(mask[list[i]]) : 0u;
+  c = __reduce_add_sync(0xFFFFFFFFu, c);
+  if ((threadIdx.x & 31u) == 0 && c) atomicAdd(&tot, c);
+  __syncthreads();
+  if (threadIdx.x == 0) sums[blockIdx.x] = tot;
+}
+
+// Level l's nodes: their place in the next list (the sums of the chunks
+// before, then a scan of the chunk), the next list itself and the refs -
+// occupied children are grid nodes or, at the last level, bricks
+// (0x40000000 | rank; map[cell] = rank).  A warp per node writes its 64 refs.
+// sums: children per chunk (null: one chunk holds the list).
+__global__ void __launch_bounds__(kListChunk)
+    expand_kernel64(const uint32_t* counts, int l, bool last, uint32_t n, const uint32_t* list,
+                    const uint64_t* mask, const uint32_t* sums, uint32_t* next, uint32_t* grids,
+                    int32_t* map) {
+  __shared__ uint64_t s_mask[kListChunk];
+  __shared__ uint32_t s_off[kListChunk], s_node[kListChunk], s_warp[kListChunk / 32], s_base;
+  const uint32_t m = list_len(counts, l), i0 = blockIdx.x * kListChunk;
+  if (i0 >= m) return;
+  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+  if (t == 0) s_base = 0;
+  __syncthreads();
+  if (sums) {
+    uint32_t b = 0;
+    for (uint32_t k = t; k < blockIdx.x; k += kListChunk) b += sums[k];
+    b = __reduce_add_sync(0xFFFFFFFFu, b);
+    if (lane == 0 && b) atomicAdd(&s_base, b);
+  }
+  const uint32_t here = m - i0 < kListChunk ? m - i0 : kListChunk;
+  const uint32_t p = t < here ? list[i0 + t] : 0u;
+  const uint64_t mk = t < here ? mask[p] : 0ull;
+  uint32_t inc = (uint32_t)__popcll(mk);
+  const uint32_t own = inc;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+    if (lane >= (uint32_t)o) inc += u;
+  }
+  if (lane == 31) s_warp[warp] = inc;
+  __syncthreads();
+  uint32_t off = s_base + inc - own;
+  for (uint32_t w = 0; w < warp; ++w) off += s_warp[w];
+  s_mask[t] = mk;
+  s_off[t] = off;
+  s_node[t] = p;
+  __syncthreads();
+  uint32_t node_base = 0, child_base = 1;  // grid nodes before this level, before the next
+  for (int k = 0; k < l; ++k) {
+    node_base = child_base;
+    child_base += counts[k + 1];
+  }
+  for (uint32_t j = warp; j < here; j += kListChunk / 32) {
+    const uint64_t bits = s_mask[j];
+    const uint32_t o = s_off[j], q = s_node[j];
+    uint32_t* g = grids + (size_t)(node_base + i0 + j) * 64;
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+      const uint32_t c = lane + 32u * h;
       uint32_t ref = 0x80000000u;
-      if (child_any[child64(list[i], n, c)]) {
-        ref = bricks ? (0x40000000u | next) : (child_base + next);
-        ++next;
+      if ((bits >> c) & 1ull) {
+        const uint32_t rank = o + (uint32_t)__popcll(bits & ((1ull << c) - 1ull));
+        const uint32_t ch = child64(q, n, c);
+        next[rank] = ch;
+        ref = last ? (0x40000000u | rank) : child_base + rank;
+        if (last && map) map[ch] = (int32_t)rank;
       }
       g[c] = ref;
     }
@@ -304,104 +400,130 @@ __device__ __forceinline__ uint16_t f16_saturating(float f) {
   return u;
 }
 
-// Pack: one warp per brick, its 729 lattice values (and RGB).  format < 0:
+// RGB of lattice point i (R in the low byte) from two aligned words, or byte by
+// byte at the array's end and where the array is not 4-byte aligned (words =
+// the whole words of the array, 0 then).
+__device__ __forceinline__ uint32_t load_rgb(const uint8_t* rgb, uint64_t i, uint64_t words) {
+  const uint64_t b = 3u * i, w = b >> 2;
+  if (w + 1 < words) {
+    const uint32_t* p = reinterpret_cast<const uint32_t*>(rgb) + w;
+    return __funnelshift_r(__ldg(p), __ldg(p + 1), ((uint32_t)b & 3u) * 8u) & 0xFFFFFFu;
+  }
+  return (uint32_t)rgb[b] | ((uint32_t)rgb[b + 1] << 8) | ((uint32_t)rgb[b + 2] << 16);
+}
+
+// Apron neighbours of a brick (index m-1 for the offset m = dx | dy<<1 |
+// dz<<2), lanes 0..6 the upper and 8..14 the lower ones.
+__device__ __forceinline__ void write_neighbors(const int32_t* map, int nb, uint32_t b, int x,
+                                                int y, int z, uint32_t lane, int32_t* up,
+                                                int32_t* dn) {
+  const int m = (int)(lane & 7u) + 1;
+  if (m > 7 || lane > 14u) return;
+  const int s = lane < 8u ? 1 : -1;
+  const int ux = x + s * (m & 1), uy = y + s * ((m >> 1) & 1), uz = z + s * (m >> 2);
+  const bool in = ux >= 0 && uy >= 0 && uz >= 0 && ux < nb && uy < nb && uz < nb;
+  const int32_t v = in ? map[((size_t)uz * nb + uy) * nb + ux] : -1;
+  (lane < 8u ? up : dn)[7 * (size_t)b + (size_t)(m - 1)] = v;
+}
+
+// Pack: one warp per brick, its 729 lattice values (and RGB).  kFormat < 0:
 // fp32 density + uint8 RGB (host container layout); else a device pool
 // format (YV_PRECISION_*), written to d_out / a_out.
-// mask (device pools, optional): the cell occupancy mask of the march (16
-// words per brick, bit (y & 3) * 8 + x of word z * 2 + (y >> 2) set where
-// trilinear cell (x, y, z) has a non-zero stored density corner), from a
-// 729-bit non-zero map of the brick's lattice the warp gathers by ballots
-// while it packs (blocks of 256 threads).
-// bits (device pools, optional, zeroed before): the brick bitmap, bit
-// (ci & 31) of word ci >> 5 set for the cell ci = (cz nb + cy) nb + cx of
-// every brick.
-__global__ void pack_bricks_kernel(Lattice g, const uint64_t* cells, uint32_t nbricks, int format,
-                                   float* dens, uint8_t* rgb, void* d_out, void* a_out,
-                                   int32_t* cell_xyz, int32_t* map, uint32_t* mask,
-                                   uint32_t* bits) {
+// The lattice offset of each of the 729 points from a brick's first is one
+// table in shared memory; loads of 8 points are issued before any is used.
+// 513^3 lattice with colours, 74 k bricks, 8-byte format: 566 us with the
+// offsets and three byte loads worked out per point.
+// Device pools (kFormat >= 0): mask is the cell occupancy mask of the march
+// (16 words per brick, cell_mask_word) of the stored densities; bits
+// (optional, zeroed before) the brick bitmap, bit (ci & 31) of word ci >> 5
+// set for the cell ci = (cz nb + cy) nb + cx of every brick; up / dn the apron
+// neighbours.  Host container: cell_xyz.
+template <int kFormat>
+__global__ void __launch_bounds__(256)
+    pack_bricks_kernel(Lattice g, const uint32_t* cells, uint32_t nbricks, uint64_t rgb_words,
+                       float* dens, uint8_t* rgb, void* d_out, void* a_out, int32_t* cell_xyz,
+                       const int32_t* map, int32_t* up, int32_t* dn, uint32_t* mask,
+                       uint32_t* bits) {
   __shared__ uint32_t nzbits[8][24];
+  __shared__ uint32_t offs[kVL3 + 7];
+  const uint32_t L = (uint32_t)g.L;
+  for (uint32_t k = threadIdx.x; k < kVL3; k += blockDim.x)
+    offs[k] = k % kVL + ((k / kVL) % kVL) * L + (k / (kVL * kVL)) * L * L;
+  __syncthreads();
   const uint32_t lane = threadIdx.x & 31u;
-  uint32_t* nz = nzbits[(threadIdx.x >> 5) & 7u];
+  uint32_t* nz = nzbits[threadIdx.x >> 5];
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const int nbs = __ffs(g.nb) - 1;
-  const bool half = format == YV_PRECISION_F16 || format == YV_PRECISION_F16_PACKED;
+  constexpr bool kHalf = kFormat == YV_PRECISION_F16 || kFormat == YV_PRECISION_F16_PACKED;
   for (uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nbricks; b += nwarps) {
-    const uint64_t c = cells[b];
-    const int cx = (int)(c & (uint64_t)(g.nb - 1)), cy = (int)((c >> nbs) & (uint64_t)(g.nb - 1)),
+    const uint32_t c = cells[b];
+    const int cx = (int)(c & (uint32_t)(g.nb - 1)), cy = (int)((c >> nbs) & (uint32_t)(g.nb - 1)),
               cz = (int)(c >> (2 * nbs));
-    if (lane == 0) {
-      cell_xyz[3 * (size_t)b] = cx;
-      cell_xyz[3 * (size_t)b + 1] = cy;
-      cell_xyz[3 * (size_t)b + 2] = cz;
-      map[c] = (int32_t)b;
-      if (bits) {
-        const uint64_t ci = ((uint64_t)cz * (uint64_t)g.nb + (uint64_t)cy) * (uint64_t)g.nb +
-                            (uint64_t)cx;
-        atomicOr(bits + (ci >> 5), 1u << (uint32_t)(ci & 31u));
+    if (kFormat < 0) {
+      if (lane == 0) {
+        cell_xyz[3 * (size_t)b] = cx;
+        cell_xyz[3 * (size_t)b + 1] = cy;
+        cell_xyz[3 * (size_t)b + 2] = cz;
       }
+    } else {
+      write_neighbors(map, g.nb, b, cx, cy, cz, lane, up, dn);
+      // the linear cell index is c itself
+      if (lane == 31 && bits) atomicOr(bits + (c >> 5), 1u << (c & 31u));
     }
-    // lattice point k = lane + 32 q; the loads of 8 points are issued before
-    // any is used
-    for (int q0 = 0; q0 < (kVL3 + 31) / 32; q0 += 8) {
+    const uint64_t first = lat(g, cx * kVB, cy * kVB, cz * kVB);
+    const float* src = g.d + first;
+    const size_t o0 = (size_t)b * kVL3;
+    for (uint32_t q0 = 0; q0 < 24u; q0 += 8u) {
       float pv[8];
+      uint32_t pc[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int k = (int)lane + 32 * (q0 + u);
-        pv[u] = k < kVL3 ? __ldg(g.d + lat(g, cx * kVB + k % kVL, cy * kVB + (k / kVL) % kVL,
-                                            cz * kVB + k / (kVL * kVL)))
-                         : 0.f;
-      }
-      if (mask) {
-        // after all 8 loads are issued: the non-zero points as stored (the
-        // fp16 formats round small values to 0), one ballot per 32
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const bool nzv = half ? (f16_saturating(pv[u]) & 0x7FFFu) != 0 : pv[u] != 0.f;
-          const uint32_t bits = __ballot_sync(0xFFFFFFFFu, nzv);
-          if (lane == 0 && q0 + u < 24) nz[q0 + u] = bits;
-        }
+      for (uint32_t u = 0; u < 8u; ++u) {
+        const uint32_t k = lane + 32u * (q0 + u);
+        const bool in = k < (uint32_t)kVL3;
+        const uint32_t o = in ? offs[k] : 0u;
+        pv[u] = in ? __ldg(src + o) : 0.f;
+        pc[u] = g.rgb ? load_rgb(g.rgb, first + o, rgb_words) : 0xFFFFFFu;
       }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int k = (int)lane + 32 * (q0 + u);
-        if (k >= kVL3) break;
-        const uint64_t src = lat(g, cx * kVB + k % kVL, cy * kVB + (k / kVL) % kVL,
-                                 cz * kVB + k / (kVL * kVL));
+      for (uint32_t u = 0; u < 8u; ++u) {
+        const uint32_t k = lane + 32u * (q0 + u);
         const float v = pv[u];
-        uint8_t r = 255, gg = 255, bb = 255;
-        if (g.rgb) {
-          r = g.rgb[3 * src];
-          gg = g.rgb[3 * src + 1];
-          bb = g.rgb[3 * src + 2];
+        const uint32_t r = pc[u] & 0xFFu, gg = (pc[u] >> 8) & 0xFFu, bb = pc[u] >> 16;
+        const uint32_t h = kHalf ? (uint32_t)f16_saturating(v) : 0u;
+        if (kFormat >= 0) {
+          // the non-zero points as stored (the fp16 formats round small
+          // values to 0); zero beyond the 729 points
+          const bool nzv = kHalf ? (h & 0x7FFFu) != 0u : v != 0.f;
+          const uint32_t bal = __ballot_sync(0xFFFFFFFFu, nzv);
+          if (lane == 0) nz[q0 + u] = bal;
         }
-        const size_t o = (size_t)b * kVL3 + (size_t)k;
-        if (format < 0) {
-          dens[o] = v;
-          rgb[3 * o] = r;
-          rgb[3 * o + 1] = gg;
-          rgb[3 * o + 2] = bb;
-        } else if (format == YV_PRECISION_F16) {
-          static_cast<uint16_t*>(d_out)[o] = f16_saturating(v);
-          static_cast<uchar4*>(a_out)[o] = make_uchar4(r, gg, bb, 255);
-        } else if (format == YV_PRECISION_F32) {
-          static_cast<float*>(d_out)[o] = v;
-          float* a = static_cast<float*>(a_out) + 3 * o;
-          a[0] = __fmul_rn((float)r, 1.0f / 255.0f);
-          a[1] = __fmul_rn((float)gg, 1.0f / 255.0f);
-          a[2] = __fmul_rn((float)bb, 1.0f / 255.0f);
-        } else if (format == YV_PRECISION_F32_PACKED) {
-          static_cast<float4*>(a_out)[o] =
-              make_float4(__fmul_rn((float)r, 1.0f / 255.0f), __fmul_rn((float)gg, 1.0f / 255.0f),
-                          __fmul_rn((float)bb, 1.0f / 255.0f), v);
-        } else {
-          static_cast<uint2*>(a_out)[o] =
-              make_uint2((uint32_t)f16_saturating(v) | ((uint32_t)r << 16) | ((uint32_t)gg << 24),
-                         (uint32_t)bb);
+        if (k < (uint32_t)kVL3) {
+          const size_t o = o0 + k;
+          if (kFormat < 0) {
+            dens[o] = v;
+            rgb[3 * o] = (uint8_t)r;
+            rgb[3 * o + 1] = (uint8_t)gg;
+            rgb[3 * o + 2] = (uint8_t)bb;
+          } else if (kFormat == YV_PRECISION_F16) {
+            static_cast<uint16_t*>(d_out)[o] = (uint16_t)h;
+            static_cast<uint32_t*>(a_out)[o] = pc[u] | 0xFF000000u;
+          } else if (kFormat == YV_PRECISION_F32) {
+            static_cast<float*>(d_out)[o] = v;
+            float* a = static_cast<float*>(a_out) + 3 * o;
+            a[0] = __fmul_rn((float)r, 1.0f / 255.0f);
+            a[1] = __fmul_rn((float)gg, 1.0f / 255.0f);
+            a[2] = __fmul_rn((float)bb, 1.0f / 255.0f);
+          } else if (kFormat == YV_PRECISION_F32_PACKED) {
+            static_cast<float4*>(a_out)[o] =
+                make_float4(__fmul_rn((float)r, 1.0f / 255.0f), __fmul_rn((float)gg, 1.0f / 255.0f),
+                            __fmul_rn((float)bb, 1.0f / 255.0f), v);
+          } else {
+            static_cast<uint2*>(a_out)[o] = make_uint2(h | (pc[u] << 16), bb);
+          }
         }
       }
     }
-    if (mask) {
-      if (lane == 0) nz[23] = 0u;  // beyond the 729 points
+    if (kFormat >= 0) {
       __syncwarp();
       if (lane < 16u) mask[(size_t)b * 16u + lane] = cell_mask_word(nz, lane);
       __syncwarp();
@@ -409,23 +531,11 @@ __global__ void pack_bricks_kernel(Lattice g, const uint64_t* cells, uint32_t nb
   }
 }
 
-// Apron neighbour tables (index m-1 for the offset m = dx | dy<<1 | dz<<2).
-__global__ void neighbors_kernel(const int32_t* cell_xyz, const int32_t* map, uint32_t nbricks,
-                                 int nb, int32_t* up, int32_t* dn) {
-  for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nbricks;
-       b += gridDim.x * blockDim.x) {
-    const int x = cell_xyz[3 * (size_t)b], y = cell_xyz[3 * (size_t)b + 1],
-              z = cell_xyz[3 * (size_t)b + 2];
-    for (int m = 1; m < 8; ++m) {
-      const int dx = m & 1, dy = (m >> 1) & 1, dz = (m >> 2) & 1;
-      const int ux = x + dx, uy = y + dy, uz = z + dz;
-      up[7 * (size_t)b + m - 1] =
-          (ux < nb && uy < nb && uz < nb) ? map[((size_t)uz * nb + uy) * nb + ux] : -1;
-      const int lx = x - dx, ly = y - dy, lz = z - dz;
-      dn[7 * (size_t)b + m - 1] =
-          (lx >= 0 && ly >= 0 && lz >= 0) ? map[((size_t)lz * nb + ly) * nb + lx] : -1;
-    }
-  }
+// Whole aligned words of the lattice's colours, 0 where the words cannot be
+// read (unaligned).
+uint64_t rgb_words(const Lattice& g) {
+  if (!g.rgb || (reinterpret_cast<uintptr_t>(g.rgb) & 3u)) return 0;
+  return 3u * g.L * g.L * g.L / 4u;
 }
 
 yv_status vbuild_fail(cudaError_t e, const char* what) {
@@ -434,99 +544,84 @@ yv_status vbuild_fail(cudaError_t e, const char* what) {
   return e == cudaErrorMemoryAllocation ? YV_ERR_OUT_OF_MEMORY : YV_ERR_CUDA;
 }
 
-// Tree of a dense lattice on the device: grid refs (ngrids x 64) and the
-// breadth-first brick cells.  Buffers come from the scratch pool.
+// Tree of a dense lattice on the device: grid refs (ngrids x 64), the
+// breadth-first brick cells and the brick of every cell (-1: none), in one
+// scratch allocation sized for a full tree.
 struct VolumeTree {
-  DevBuf grids, cells;  // uint32 grids[ngrids*64], uint64 cells[nbricks]
+  DevBuf mem;
+  uint32_t* grids = nullptr;
+  uint32_t* cells = nullptr;
+  int32_t* map = nullptr;
   uint32_t ngrids = 0, nbricks = 0;
 };
 
 yv_status build_volume_tree(const Lattice& g, int levels, cudaStream_t s, VolumeTree& t) {
-  cudaError_t e;
-  std::vector<DevBuf> any((size_t)levels + 1);
-  for (int l = 0; l <= levels; ++l) {
-    const uint64_t n = 1ull << (2 * l);
-    if ((e = any[(size_t)l].alloc(n * n * n, s)) != cudaSuccess) return vbuild_fail(e, "alloc");
+  const uint64_t NW = g.nb >= 32 ? (uint64_t)g.nb / 32 : 1;
+  const uint64_t cells = (uint64_t)g.nb * g.nb * g.nb;
+  // the parts of the scratch, 256-byte aligned: node masks and lists per
+  // level, sums of the largest list, grid refs, cell map, row bits, counts
+  uint64_t total = 0, max_grids = 0;
+  auto part = [&](uint64_t bytes) {
+    const uint64_t at = total;
+    total += (bytes + 255u) & ~255ull;
+    return at;
+  };
+  uint64_t mask_at[5], list_at[6];
+  for (int l = 0; l < levels; ++l) {
+    mask_at[l] = part((1ull << (6 * l)) * 8);
+    max_grids += 1ull << (6 * l);
   }
-  // occupied nodes per level (counted by the mark and fold passes, read
-  // back once): the breadth-first lists below need no host read per level
-  DevBuf dc;
-  if ((e = dc.alloc((size_t)(levels + 1) * 4, s)) != cudaSuccess ||
-      (e = cudaMemsetAsync(dc.p, 0, (size_t)(levels + 1) * 4, s)) != cudaSuccess)
-    return vbuild_fail(e, "alloc");
-  {
-    const uint64_t NW = g.nb >= 32 ? (uint64_t)g.nb / 32 : 1;
-    DevBuf rows;
-    if ((e = rows.alloc(g.L * g.L * NW * 4, s)) != cudaSuccess) return vbuild_fail(e, "alloc");
-    if (g.nb >= 16 && NW <= kFlatMaxNW && (reinterpret_cast<uintptr_t>(g.d) & 15u) == 0)
-      mark_rows_flat_kernel<<<grid_for((g.L * g.L + 3) / 4 * 32), 256, 0, s>>>(
-          g, rows.as<uint32_t>());
-    else
-      mark_rows_kernel<<<grid_for(g.L * g.L * 32), 256, 0, s>>>(g, rows.as<uint32_t>());
-    mark_cells_from_rows_kernel<<<grid_for(NW * g.nb * g.nb), 256, 0, s>>>(
-        g, rows.as<uint32_t>(), any[(size_t)levels].as<uint8_t>(), dc.as<uint32_t>() + levels);
-  }
-  for (int l = levels - 1; l >= 0; --l) {
+  for (int l = 0; l <= levels; ++l) list_at[l] = part((1ull << (6 * l)) * 4);
+  const uint64_t sums_at = part(((1ull << (6 * (levels - 1))) / kListChunk + 1) * 4);
+  const uint64_t grids_at = part(max_grids * 256);
+  const uint64_t map_at = part(cells * 4);
+  const uint64_t rows_at = part(g.L * g.L * NW * 4);
+  const uint64_t counts_at = part(256);
+  cudaError_t e = t.mem.alloc(total, s);
+  if (e != cudaSuccess) return vbuild_fail(e, "alloc");
+  char* mem = t.mem.as<char>();
+  auto mask = [&](int l) { return reinterpret_cast<uint64_t*>(mem + mask_at[l]); };
+  auto list = [&](int l) { return reinterpret_cast<uint32_t*>(mem + list_at[l]); };
+  uint32_t* sums = reinterpret_cast<uint32_t*>(mem + sums_at);
+  uint32_t* rows = reinterpret_cast<uint32_t*>(mem + rows_at);
+  uint32_t* counts = reinterpret_cast<uint32_t*>(mem + counts_at);
+  t.grids = reinterpret_cast<uint32_t*>(mem + grids_at);
+  t.cells = list(levels);
+  t.map = reinterpret_cast<int32_t*>(mem + map_at);
+  if ((e = cudaMemsetAsync(counts, 0, 256, s)) != cudaSuccess ||
+      (e = cudaMemsetAsync(list(0), 0, 4, s)) != cudaSuccess ||
+      (e = cudaMemsetAsync(t.map, 0xFF, cells * 4, s)) != cudaSuccess)
+    return vbuild_fail(e, "clear");
+  if (g.nb >= 16 && NW <= kFlatMaxNW && (reinterpret_cast<uintptr_t>(g.d) & 15u) == 0)
+    mark_rows_flat_kernel<<<grid_for((g.L * g.L + 3) / 4 * 32), 256, 0, s>>>(g, rows);
+  else
+    mark_rows_kernel<<<grid_for(g.L * g.L * 32), 256, 0, s>>>(g, rows);
+  // a warp per word and 4x4 square of cells
+  const uint64_t n4 = (uint64_t)g.nb / 4;
+  mark_nodes_kernel<<<(unsigned)((NW * n4 * n4 + 7) / 8), 256, 0, s>>>(
+      g, rows, mask(levels - 1), counts + (levels > 1 ? levels - 1 : 8), counts + levels);
+  for (int l = levels - 2; l >= 0; --l) {
     const uint32_t n = 1u << (2 * l);
-    fold64_kernel<<<grid_for((uint64_t)n * n * n), 256, 0, s>>>(
-        any[(size_t)l + 1].as<uint8_t>(), n, any[(size_t)l].as<uint8_t>(),
-        dc.as<uint32_t>() + l);
+    fold_masks_kernel<<<(unsigned)(((uint64_t)n * n * n + 7) / 8), 256, 0, s>>>(
+        mask(l + 1), n, mask(l), counts + (l > 0 ? l : 8));  // [8]: not read
   }
-  std::vector<uint32_t> occ((size_t)levels + 1, 0);
+  for (int l = 0; l < levels; ++l) {
+    const uint32_t chunks = (uint32_t)(((1ull << (6 * l)) + kListChunk - 1) / kListChunk);
+    if (chunks > 1)
+      child_sums_kernel<<<chunks, kListChunk, 0, s>>>(counts, l, list(l), mask(l), sums);
+    expand_kernel64<<<chunks, kListChunk, 0, s>>>(counts, l, l == levels - 1, 1u << (2 * l),
+                                                  list(l), mask(l), chunks > 1 ? sums : nullptr,
+                                                  list(l + 1), t.grids, t.map);
+  }
+  uint32_t hc[8] = {};
   if ((e = cudaGetLastError()) != cudaSuccess ||
-      (e = cudaMemcpyAsync(occ.data(), dc.p, (size_t)(levels + 1) * 4, cudaMemcpyDeviceToHost,
-                           s)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(hc, counts, sizeof(hc), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
       (e = cudaStreamSynchronize(s)) != cudaSuccess)
-    return vbuild_fail(e, "mark");
-  // breadth-first lists: level 0 = the root (always a grid node)
-  std::vector<DevBuf> list((size_t)levels + 1), offs((size_t)levels);
-  std::vector<uint32_t> m((size_t)levels + 1, 0), base((size_t)levels + 1, 0);
-  if ((e = list[0].alloc(8, s)) != cudaSuccess ||
-      (e = cudaMemsetAsync(list[0].p, 0, 8, s)) != cudaSuccess)
-    return vbuild_fail(e, "alloc");
-  m[0] = 1;
-  for (int l = 0; l < levels; ++l) {
-    const uint32_t n = 1u << (2 * l);
-    DevBuf counts;
-    if ((e = counts.alloc((size_t)m[(size_t)l] * 4, s)) != cudaSuccess ||
-        (e = offs[(size_t)l].alloc((size_t)m[(size_t)l] * 4, s)) != cudaSuccess)
-      return vbuild_fail(e, "alloc");
-    if (m[(size_t)l])
-      count64_kernel<<<grid_for(m[(size_t)l]), 256, 0, s>>>(
-          list[(size_t)l].as<uint64_t>(), m[(size_t)l], any[(size_t)l + 1].as<uint8_t>(), n,
-          counts.as<uint32_t>());
-    if ((e = cudaGetLastError()) != cudaSuccess ||
-        (e = exclusive_scan(counts.as<uint32_t>(), offs[(size_t)l].as<uint32_t>(),
-                            m[(size_t)l], nullptr, s)) != cudaSuccess)
-      return vbuild_fail(e, "scan");
-    const uint32_t total = occ[(size_t)l + 1];  // the scanned total
-    base[(size_t)l + 1] = base[(size_t)l] + m[(size_t)l];
-    m[(size_t)l + 1] = total;
-    if ((e = list[(size_t)l + 1].alloc((size_t)(total ? total : 1) * 8, s)) != cudaSuccess)
-      return vbuild_fail(e, "alloc");
-    if (m[(size_t)l])
-      expand64_kernel<<<grid_for(m[(size_t)l]), 256, 0, s>>>(
-          list[(size_t)l].as<uint64_t>(), m[(size_t)l], any[(size_t)l + 1].as<uint8_t>(), n,
-          offs[(size_t)l].as<uint32_t>(), list[(size_t)l + 1].as<uint64_t>());
-    if ((e = cudaGetLastError()) != cudaSuccess) return vbuild_fail(e, "expand");
-  }
-  // grid nodes: levels 0..levels-1; bricks: the last list
-  t.ngrids = base[(size_t)levels];
-  t.nbricks = m[(size_t)levels];
-  if ((e = t.grids.alloc((size_t)t.ngrids * 256, s)) != cudaSuccess)
-    return vbuild_fail(e, "alloc");
-  for (int l = 0; l < levels; ++l) {
-    if (!m[(size_t)l]) continue;
-    const bool last = l == levels - 1;
-    emit_grids_kernel<<<grid_for(m[(size_t)l]), 256, 0, s>>>(
-        list[(size_t)l].as<uint64_t>(), m[(size_t)l], any[(size_t)l + 1].as<uint8_t>(),
-        1u << (2 * l), offs[(size_t)l].as<uint32_t>(), base[(size_t)l],
-        last ? 0u : base[(size_t)l + 1], last, t.grids.as<uint32_t>());
-  }
-  if ((e = cudaGetLastError()) != cudaSuccess) return vbuild_fail(e, "grids");
-  // hand over the brick list
-  std::swap(t.cells.p, list[(size_t)levels].p);
-  t.cells.s = s;
+    return vbuild_fail(e, "tree");
+  // grid nodes: the root and the occupied nodes of levels 1..levels-1
+  t.ngrids = 1;
+  for (int l = 1; l < levels; ++l) t.ngrids += hc[l];
+  t.nbricks = hc[levels];
   return YV_OK;
 }
 
@@ -557,23 +652,21 @@ yv_status yv_volume_build_dense(const float* density, const uint8_t* rgb, int32_
   yv_status st = build_volume_tree(g, levels, s, t);
   if (st != YV_OK) return st;
   const size_t n = (size_t)t.nbricks * kVL3;
-  DevBuf dens, col, cxyz, map;
-  const uint64_t cells = (uint64_t)g.nb * g.nb * g.nb;
+  DevBuf dens, col, cxyz;
   cudaError_t e;
   if ((e = dens.alloc(n * 4, s)) != cudaSuccess || (e = col.alloc(n * 3, s)) != cudaSuccess ||
-      (e = cxyz.alloc((size_t)t.nbricks * 12, s)) != cudaSuccess ||
-      (e = map.alloc(cells * 4, s)) != cudaSuccess)
+      (e = cxyz.alloc((size_t)t.nbricks * 12, s)) != cudaSuccess)
     return vbuild_fail(e, "alloc");
   if (t.nbricks)
-    pack_bricks_kernel<<<grid_for((uint64_t)t.nbricks * 32), 256, 0, s>>>(
-        g, t.cells.as<uint64_t>(), t.nbricks, -1, dens.as<float>(), col.as<uint8_t>(), nullptr,
-        nullptr, cxyz.as<int32_t>(), map.as<int32_t>(), nullptr, nullptr);
+    pack_bricks_kernel<-1><<<grid_for((uint64_t)t.nbricks * 32), 256, 0, s>>>(
+        g, t.cells, t.nbricks, rgb_words(g), dens.as<float>(), col.as<uint8_t>(), nullptr,
+        nullptr, cxyz.as<int32_t>(), nullptr, nullptr, nullptr, nullptr, nullptr);
   if ((e = cudaGetLastError()) != cudaSuccess) return vbuild_fail(e, "pack");
   std::vector<uint32_t> grids((size_t)t.ngrids * 64);
   std::vector<float> hd(n);
   std::vector<uint8_t> hc(n * 3);
   std::vector<int32_t> hcell((size_t)t.nbricks * 3);
-  if ((e = cudaMemcpyAsync(grids.data(), t.grids.p, grids.size() * 4, cudaMemcpyDeviceToHost,
+  if ((e = cudaMemcpyAsync(grids.data(), t.grids, grids.size() * 4, cudaMemcpyDeviceToHost,
                            s)) != cudaSuccess ||
       (n && (e = cudaMemcpyAsync(hd.data(), dens.p, n * 4, cudaMemcpyDeviceToHost, s)) !=
                 cudaSuccess) ||
@@ -605,7 +698,6 @@ yv_status upload_dense(const float* density, const uint8_t* rgb, int32_t levels,
   yv_status st = build_volume_tree(g, levels, s, t);
   if (st != YV_OK) return st;
   const size_t n = (size_t)t.nbricks * kVL3;
-  const uint64_t cells = (uint64_t)g.nb * g.nb * g.nb;
   size_t dbytes = 0, abytes = 0;
   switch (precision) {
     case YV_PRECISION_F16: dbytes = n * 2; abytes = n * 4; break;
@@ -648,21 +740,18 @@ yv_status upload_dense(const float* density, const uint8_t* rgb, int32_t levels,
       if (e == cudaSuccess && levels <= 4) bits = mask + (size_t)t.nbricks * 16u;
     }
   }
-  DevBuf cxyz, map;
-  if (e == cudaSuccess) e = cxyz.alloc((size_t)t.nbricks * 12, s);
-  if (e == cudaSuccess) e = map.alloc(cells * 4, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(map.p, 0xFF, cells * 4, s);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(mem[0], t.grids.p, bytes[0], cudaMemcpyDeviceToDevice, s);
+    e = cudaMemcpyAsync(mem[0], t.grids, bytes[0], cudaMemcpyDeviceToDevice, s);
   if (e == cudaSuccess && bits)
     e = cudaMemsetAsync(bits, 0, (size_t)YV_BRICK_BITS_WORDS(levels) * 4u, s);
   if (e == cudaSuccess && t.nbricks) {
-    pack_bricks_kernel<<<grid_for((uint64_t)t.nbricks * 32), 256, 0, s>>>(
-        g, t.cells.as<uint64_t>(), t.nbricks, precision, nullptr, nullptr, mem[1], mem[2],
-        cxyz.as<int32_t>(), map.as<int32_t>(), mask, bits);
-    neighbors_kernel<<<grid_for(t.nbricks), 256, 0, s>>>(
-        cxyz.as<int32_t>(), map.as<int32_t>(), t.nbricks, g.nb, static_cast<int32_t*>(mem[3]),
-        static_cast<int32_t*>(mem[4]));
+    auto kern = precision == YV_PRECISION_F16          ? pack_bricks_kernel<YV_PRECISION_F16>
+                : precision == YV_PRECISION_F32        ? pack_bricks_kernel<YV_PRECISION_F32>
+                : precision == YV_PRECISION_F32_PACKED ? pack_bricks_kernel<YV_PRECISION_F32_PACKED>
+                                                       : pack_bricks_kernel<YV_PRECISION_F16_PACKED>;
+    kern<<<grid_for((uint64_t)t.nbricks * 32), 256, 0, s>>>(
+        g, t.cells, t.nbricks, rgb_words(g), nullptr, nullptr, mem[1], mem[2], nullptr, t.map,
+        static_cast<int32_t*>(mem[3]), static_cast<int32_t*>(mem[4]), mask, bits);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {
