@@ -110,12 +110,16 @@ __global__ void mark_rows_kernel(Lattice g, uint32_t* R) {
 // warp's 128 points touch at most two rows): the rows
 // in groups of 4 (4 L floats start on a 16-byte boundary, L = 8 nb + 1 being
 // odd only shifts the rows inside a group), read as float4 by one warp per
-// group, 128 points per warp load.  A lane marks the cells of its 4 points
-// (own cell x >> 3, apron cell x / 8 - 1 for x a non-zero multiple of 8) in
-// a 32-bit window of cells of the warp's row; one warp OR reduction per row
-// the load touches (at most 2), and lane 0 merges it into the group's row
-// words in shared memory.  Same R as mark_rows_kernel.
+// group, 128 points per warp load, the next loads under way.  A lane marks the
+// cells of its 4 points (own cell x >> 3, apron cell x / 8 - 1 for x a
+// non-zero multiple of 8) in a 32-bit window of cells of the warp's row; one
+// warp OR reduction per row the load touches (at most 2), and lane 0 merges it
+// into the group's row words in shared memory.  A bit past the last cell (its
+// apron point) is dropped with the words or masked at the end.  Same R as
+// mark_rows_kernel.  513^3: 155 us with per-point tests of row and cell, 138 us
+// one load at a time, 122 us with 4 under way (128 with 2 or 8).
 constexpr uint32_t kFlatMaxNW = 8;
+constexpr uint32_t kFlatAhead = 4;  // loads a lane has under way
 
 __global__ void mark_rows_flat_kernel(Lattice g, uint32_t* R) {
   __shared__ uint32_t acc_all[8][4][kFlatMaxNW];
@@ -140,87 +144,60 @@ __global__ void mark_rows_flat_kernel(Lattice g, uint32_t* R) {
     // row and x of the warp's first point, advanced by 128 points a step
     // (L > 128: at most one row boundary per step)
     uint32_t ra = 0, xs = 0;
-    for (uint32_t f0 = 0; f0 < n4; f0 += 32u) {
-      const uint32_t f = f0 + lane;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (4u * f + 3u < nfl) {
-        v = __ldg(src + f);
-      } else if (f < n4) {
-        // the group's (and the lattice's) last points: no read past them
-        const float* s1 = reinterpret_cast<const float*>(src) + 4u * f;
-        const uint32_t left = nfl - 4u * f;
-        v.x = __ldg(s1);
-        if (left > 1u) v.y = __ldg(s1 + 1);
-        if (left > 2u) v.z = __ldg(s1 + 2);
+    for (uint32_t f1 = 0; f1 < n4; f1 += 32u * kFlatAhead) {
+      float4 ahead[kFlatAhead];
+#pragma unroll
+      for (uint32_t u = 0; u < kFlatAhead; ++u) {
+        const uint32_t f = f1 + 32u * u + lane;
+        ahead[u] = 4u * f + 3u < nfl ? __ldg(src + f) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      if (xs + 128u <= L && 128u + 4u * f0 <= nfl) {
-        // all 128 points in row ra (uniform): the lane's 4 points shifted to
-        // their place among the 8 of their cell; bit 0 is also the previous
-        // cell's apron, bit 8 the first point of the next cell and this
-        // one's apron
-        const uint32_t q = (xs & 7u) + 4u * lane;
+#pragma unroll
+      for (uint32_t u = 0; u < kFlatAhead; ++u) {
+        const uint32_t f0 = f1 + 32u * u, f = f0 + lane;
+        if (f0 >= n4) break;
+        float4 v = ahead[u];
+        if (4u * f + 3u >= nfl && f < n4) {
+          // the group's (and the lattice's) last points: no read past them
+          const float* s1 = reinterpret_cast<const float*>(src) + 4u * f;
+          const uint32_t left = nfl - 4u * f;
+          v.x = __ldg(s1);
+          if (left > 1u) v.y = __ldg(s1 + 1);
+          if (left > 2u) v.z = __ldg(s1 + 2);
+        }
+        // the lane's 4 points, the first `own` of them in row ra, the rest in
+        // the next; shifted to their place among the 8 of their cell, bit 0 is
+        // also the previous cell's apron, bit 8 the next cell's first point and
+        // this one's apron.  Window bit 0: the cell before the warp's first
+        // (row ra), cell -1 (the next row).
         const uint32_t nib = (v.x != 0.f ? 1u : 0u) | (v.y != 0.f ? 2u : 0u) |
                              (v.z != 0.f ? 4u : 0u) | (v.w != 0.f ? 8u : 0u);
-        const uint32_t p = nib << (q & 7u);
-        const uint32_t bits = (p & 1u) | ((p & 0x1FFu) ? 2u : 0u) | ((p >> 8) ? 4u : 0u);
-        // window bit 0: the cell before the warp's first
-        const uint32_t win = __reduce_or_sync(0xFFFFFFFFu, bits << (q >> 3));
-        if (lane == 0 && win) {
-          const uint32_t c = xs >> 3;
-          const uint64_t sft = c ? (uint64_t)win << ((c - 1u) & 31u) : (uint64_t)(win >> 1);
-          const uint32_t w = c ? (c - 1u) >> 5 : 0u;
-          if (w < NW) acc[ra][w] |= (uint32_t)sft;
-          if (w + 1 < NW) acc[ra][w + 1] |= (uint32_t)(sft >> 32);
+        const uint32_t xl = xs + 4u * lane;
+        const uint32_t own = xl >= L ? 0u : (L - xl < 4u ? L - xl : 4u);
+        {
+          const uint32_t q = (xs & 7u) + 4u * lane;
+          const uint32_t p = (nib & ((1u << own) - 1u)) << (q & 7u);
+          const uint32_t bits = (p & 1u) | ((p & 0x1FFu) ? 2u : 0u) | ((p >> 8) ? 4u : 0u);
+          const uint32_t win = __reduce_or_sync(0xFFFFFFFFu, bits << (q >> 3));
+          if (lane == 0 && win) {
+            const uint32_t c = xs >> 3;
+            const uint64_t sft = c ? (uint64_t)win << ((c - 1u) & 31u) : (uint64_t)(win >> 1);
+            const uint32_t w = c ? (c - 1u) >> 5 : 0u;
+            if (w < NW) acc[ra][w] |= (uint32_t)sft;
+            if (w + 1 < NW) acc[ra][w + 1] |= (uint32_t)(sft >> 32);
+          }
+        }
+        if (xs + 128u > L) {  // the whole warp
+          const uint32_t q = xl >= L ? xl - L : 0u;
+          const uint32_t p = (nib >> own) << (q & 7u);
+          const uint32_t bits = (p & 1u) | ((p & 0x1FFu) ? 2u : 0u) | ((p >> 8) ? 4u : 0u);
+          const uint32_t win = __reduce_or_sync(0xFFFFFFFFu, bits << (q >> 3));
+          if (lane == 0 && win && ra + 1u < nrows) acc[ra + 1u][0] |= win >> 1;
         }
         xs += 128u;
         if (xs >= L) {
           xs -= L;
           ++ra;
         }
-        continue;
-      }
-      // the warp's 128 points: rows ra (first point) .. ra + 1
-      const int c_lo = (int)(xs >> 3) - 1;  // window: cells c_lo .. c_lo + 31
-      const uint32_t rb = ra + 1;           // cells -1..30 of the next row
-      const uint32_t xl = xs + 4u * lane;   // x of the lane's first point in row ra
-      uint32_t wa = 0, wb = 0;
-      const float e[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t i = 4u * f + (uint32_t)k;
-        if (e[k] == 0.f || i >= nfl) continue;
-        uint32_t x = xl + (uint32_t)k;
-        const bool next_row = x >= L;
-        if (next_row) x -= L;
-        const uint32_t own = x >> 3;  // x = 8 nb: no own cell
-        uint32_t bits = 0;
-        if (own < nb) bits |= 2u;                  // cell own
-        if ((x & 7u) == 0u && x > 0u) bits |= 1u;  // apron of cell own - 1
-        if (!next_row) {
-          wa |= bits << (own - (uint32_t)(c_lo + 1));
-        } else {
-          wb |= bits << own;  // window of row rb starts at cell -1
-        }
-      }
-      wa = __reduce_or_sync(0xFFFFFFFFu, wa);
-      wb = __reduce_or_sync(0xFFFFFFFFu, wb);
-      if (lane == 0) {
-        // window bit b = cell base + b: row ra base c_lo, row rb base -1
-        if (wa) {
-          int c0 = c_lo;
-          uint64_t s = wa;
-          if (c0 < 0) { s >>= 1; c0 = 0; }
-          s <<= (c0 & 31);
-          const uint32_t w = (uint32_t)c0 >> 5;
-          if (w < NW) acc[ra][w] |= (uint32_t)s;
-          if (w + 1 < NW) acc[ra][w + 1] |= (uint32_t)(s >> 32);
-        }
-        if (wb && rb < nrows) acc[rb][0] |= wb >> 1;
-      }
-      xs += 128u;
-      if (xs >= L) {
-        xs -= L;
-        ++ra;
       }
     }
     __syncwarp();
@@ -432,14 +409,16 @@ __device__ __forceinline__ void write_neighbors(const int32_t* map, int nb, uint
 // The lattice offset of each of the 729 points from a brick's first is one
 // table in shared memory; loads of 8 points are issued before any is used.
 // 513^3 lattice with colours, 74 k bricks, 8-byte format: 566 us with the
-// offsets and three byte loads worked out per point.
+// offsets and three byte loads worked out per point, 283 us so, 235 us with
+// registers for 6 blocks an SM (4 without the bound; 8 spill: 270 us): bound
+// by the latency of its loads.
 // Device pools (kFormat >= 0): mask is the cell occupancy mask of the march
 // (16 words per brick, cell_mask_word) of the stored densities; bits
 // (optional, zeroed before) the brick bitmap, bit (ci & 31) of word ci >> 5
 // set for the cell ci = (cz nb + cy) nb + cx of every brick; up / dn the apron
 // neighbours.  Host container: cell_xyz.
 template <int kFormat>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 6)
     pack_bricks_kernel(Lattice g, const uint32_t* cells, uint32_t nbricks, uint64_t rgb_words,
                        float* dens, uint8_t* rgb, void* d_out, void* a_out, int32_t* cell_xyz,
                        const int32_t* map, int32_t* up, int32_t* dn, uint32_t* mask,
