@@ -115,3 +115,31 @@ def test_register_budgets_agree(yoxel_mod, precision):
     for k in (0, 31):
         assert torch.equal(yoxel_mod.render_volume(gv.desc(), [cams[k]], 67, 43)[0], many[k])
     assert float(many[..., 3].max()) > 0.1
+
+
+@pytest.mark.parametrize("special", [None, float("inf"), float("nan")])
+def test_gradient_scratch_layouts_agree(yoxel_mod, special):
+    """64 frames keep edge records in the gradient scratch, one frame points;
+    the other 63 frames have no gradient."""
+    import torch
+    tv = volume(yoxel_mod, 1, "sparse")
+    cam = yoxel_mod.sphere_cameras(5)[2]
+    rng = np.random.default_rng(4)
+    one = torch.from_numpy(rng.standard_normal((1, 40, 40, 4)).astype(np.float32)).cuda()
+    if special is not None:
+        one[0, 17, 21, 1] = special
+    many = torch.zeros((64, 40, 40, 4), device="cuda")
+    many[0] = one[0]
+    out = []
+    for cams, g in (([cam], one), ([cam] * 64, many)):
+        den = tv["density"].clone().requires_grad_(True)
+        alb = tv["albedo"].clone().requires_grad_(True)
+        rgba = yoxel_mod.volume_march(den, alb, tv, cams, 40, 40)
+        out.append(torch.autograd.grad(rgba, (den, alb), g))
+    for a, b in zip(*out):
+        assert torch.equal(a.isfinite(), b.isfinite())
+        a, b = a.nan_to_num(0.0, 0.0, 0.0), b.nan_to_num(0.0, 0.0, 0.0)
+        # FP32 sums of at most some hundred terms per point in another order:
+        # sqrt(256) 2^-24 = 1e-6
+        assert float((a - b).norm() / b.norm()) < 1e-6
+        assert float(b.norm()) > 0

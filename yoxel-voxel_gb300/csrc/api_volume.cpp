@@ -442,9 +442,9 @@ yv_status yv_volume_render_rgba8(const yv_volume_device* vol, const yv_camera* c
 
 }  // extern "C"
 
-// The adjoint of the ncams frames into a packed (albedo rgb, density) float4
-// per lattice point - one 16-byte atomic per corner - taken from the
-// stream-ordered pool, then `finish(args, packed)` on the same stream.
+// The adjoint of the ncams frames into a gradient scratch taken from the
+// stream-ordered pool (16 bytes per lattice point, 32 with edge records), then
+// `finish(args, scratch, edges)` on the same stream.
 template <class Finish>
 static yv_status run_backward(const yv_volume_device* vol, const yv_camera* cams, int32_t ncams,
                               int32_t width, int32_t height, const yv_march_params* mp,
@@ -459,23 +459,34 @@ static yv_status run_backward(const yv_volume_device* vol, const yv_camera* cams
   }
   const size_t px = (size_t)width * (size_t)height;
   const size_t npts = (size_t)vol->nbricks * 729u;
-  float4* packed = nullptr;
+  float4* scratch = nullptr;
+  a->ncams = ncams < kMaxVolumeCams ? ncams : kMaxVolumeCams;
+  // edge records while the pool keeps a scratch of their size between calls
+  // with room to spare (it holds on to 4 GiB), and where they can be had
+  size_t bytes = npts * sizeof(float4);
+  bool edges = bytes <= (1ull << 30) && backward_uses_edges(*a);
   cudaError_t e = cudaSuccess;
   if (npts) {
-    e = scratch_alloc(reinterpret_cast<void**>(&packed), npts * sizeof(float4), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(packed, 0, npts * sizeof(float4), s);
+    e = scratch_alloc(reinterpret_cast<void**>(&scratch), bytes * (edges ? 2u : 1u), s);
+    if (e == cudaErrorMemoryAllocation && edges) {
+      cudaGetLastError();
+      edges = false;
+      e = scratch_alloc(reinterpret_cast<void**>(&scratch), bytes, s);
+    }
+    if (edges) bytes *= 2u;
+    if (e == cudaSuccess) e = cudaMemsetAsync(scratch, 0, bytes, s);
   }
   for (int c0 = 0; c0 < ncams && e == cudaSuccess && npts; c0 += kMaxVolumeCams) {
     const int n = ncams - c0 < kMaxVolumeCams ? ncams - c0 : kMaxVolumeCams;
     set_cams(a, cams + c0, n);
     a->rgba_fwd = rgba + (size_t)c0 * px * 4;
     a->grad_rgba = grad_rgba + (size_t)c0 * px * 4;
-    a->grad_packed = packed;
-    e = launch_volume_backward(*a, s);
+    a->grad_scratch = scratch;
+    e = launch_volume_backward(*a, edges, s);
   }
-  if (e == cudaSuccess && npts) e = finish(*a, packed);
-  if (packed) {
-    cudaError_t ef = scratch_free(packed, s);
+  if (e == cudaSuccess && npts) e = finish(*a, scratch, edges);
+  if (scratch) {
+    cudaError_t ef = scratch_free(scratch, s);
     if (e == cudaSuccess) e = ef;
   }
   delete a;
@@ -491,9 +502,9 @@ yv_status yv_volume_backward(const yv_volume_device* vol, const yv_camera* cams,
   if (!grad_density || !grad_albedo) return YV_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   return run_backward(vol, cams, ncams, width, height, mp, rgba, grad_rgba, s,
-                      [&](const VolumeArgs& a, const float4* packed) {
-                        return launch_unpack_grads(packed, a.v.nbricks * 729u, grad_density,
-                                                   grad_albedo, s);
+                      [&](const VolumeArgs& a, const float4* scratch, bool edges) {
+                        return launch_unpack_grads(scratch, edges, a.v.nbricks * 729u,
+                                                   grad_density, grad_albedo, s);
                       });
 }
 
@@ -540,8 +551,9 @@ yv_status yv_volume_train_backward(const yv_volume_device* vol, const yv_camera*
     return YV_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   return run_backward(vol, cams, ncams, width, height, mp, rgba, grad_rgba, s,
-                      [&](const VolumeArgs& a, const float4* packed) {
-                        return launch_fold_packed(a, packed, grad_density, grad_albedo, s);
+                      [&](const VolumeArgs& a, const float4* scratch, bool edges) {
+                        return launch_fold_grads(a, scratch, edges, grad_density, grad_albedo,
+                                                 s);
                       });
 }
 

@@ -132,17 +132,31 @@ __device__ __forceinline__ float sample_dsigma(const VolumeArgs* a, float gc, fl
 
 // Per-lane coalescing of corner gradients while consecutive samples share
 // a trilinear cell: per corner, sum w_j dsigma (density) and sum w_j T alpha
-// (colour, scaled by g at the flush), flushed with one 16-byte vector atomic
-// per corner into the packed (albedo rgb, density) gradient of the lattice
-// point.  The first sample of a cell sets the accumulators.  (Carrying the 4
-// shared corners over a face-adjacent move halves the atomics but measured
-// 1.3x slower: the per-axis cases diverge within a warp.)
+// (colour, scaled by g at the flush).  The first sample of a cell sets the
+// accumulators.  (Carrying the 4 shared corners over a face-adjacent move
+// halves the atomics but measured 1.3x slower: the per-axis cases diverge
+// within a warp.)
+//
+// Flush: an atomic costs by the request, not by the byte.  With kEdges the
+// gradient scratch holds 8 floats per lattice point p for the edge (p, p + 1 in
+// x):
+//   {density p, density p + 1, r p, g p, b p, r p + 1, g p + 1, b p + 1}
+// One 8-byte atomic per edge carries the densities of both its ends: 4 for a
+// cell that the ray crossed at alpha 0 (most cells), 8 of 16 bytes for one
+// with colour.  Without, 4 floats (albedo rgb, density) per point and 8 atomics
+// of 16 bytes for either.  64-camera fitting step of a 128^3 volume 8.46 -> 7.51
+// ms with edges; a launch that does not fill the GPU is bound by its longest
+// warp, not by atomics, and keeps the smaller scratch (4 cameras at 64x64: 494
+// us, 542 with edges).
+template <bool kEdges>
 struct GradVis {
   const VolumeArgs* a;
   float g[4];   // dL/d(r,g,b,a) of this ray
   float gout;   // g . (forward output of this ray)
   float gb;     // g . (r, g, b, A) composited before the current sample
   uint32_t base;
+  float wsum;    // sum of T alpha over the cell's samples; NaN where g is not
+                 // finite (0 x g is not 0 then)
   f32x2 acc[8];  // (density, colour weight)
   __device__ __forceinline__ void init() {
     base = 0xFFFFFFFFu;
@@ -150,12 +164,35 @@ struct GradVis {
   }
   __device__ __forceinline__ void flush() {
     if (base == 0xFFFFFFFFu) return;
+    if (!kEdges) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float gd, gw;
-      unpack2(acc[j], gd, gw);
-      atomicAdd(a->grad_packed + base + corner_offset(j),
-                make_float4(fmul(g[0], gw), fmul(g[1], gw), fmul(g[2], gw), gd));
+      for (int j = 0; j < 8; ++j) {
+        float d, w;
+        unpack2(acc[j], d, w);
+        atomicAdd(a->grad_scratch + base + corner_offset(j),
+                  make_float4(fmul(g[0], w), fmul(g[1], w), fmul(g[2], w), d));
+      }
+      return;
+    }
+    float4* p = a->grad_scratch + 2 * (size_t)base;
+    if (wsum == 0.f) {
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) {
+        float d0, d1, w;
+        unpack2(acc[j], d0, w);
+        unpack2(acc[j + 1], d1, w);
+        atomicAdd(reinterpret_cast<float2*>(p + 2u * corner_offset(j)), make_float2(d0, d1));
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) {
+        float d0, d1, w0, w1;
+        unpack2(acc[j], d0, w0);
+        unpack2(acc[j + 1], d1, w1);
+        atomicAdd(p + 2u * corner_offset(j), make_float4(d0, d1, fmul(g[0], w0), fmul(g[1], w0)));
+        atomicAdd(p + 2u * corner_offset(j) + 1,
+                  make_float4(fmul(g[2], w0), fmul(g[0], w1), fmul(g[1], w1), fmul(g[2], w1)));
+      }
     }
   }
   __device__ __forceinline__ void operator()(const SampleCtx& s, float T, float w) {
@@ -166,17 +203,39 @@ struct GradVis {
     if (s.base != base) {
       flush();
       base = s.base;
+      if (kEdges) wsum = ffma(0.f, fadd(fadd(g[0], g[1]), g[2]), w);
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] = mul2(pack2(s.w[j], s.w[j]), v);
     } else {
+      if (kEdges) wsum = fadd(wsum, w);
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] = fma2(pack2(s.w[j], s.w[j]), v, acc[j]);
     }
   }
 };
 
+// Gradient (albedo rgb, density) of a lattice point, x its place in its row:
+// with kEdges what its own edge and the edge before it hold for it.
+template <bool kEdges>
+__device__ __forceinline__ float4 point_grad(const float4* __restrict__ p, size_t point, int x) {
+  if (!kEdges) return __ldg(p + point);
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (x < 8) {
+    const float4 a = __ldg(p + 2 * point), b = __ldg(p + 2 * point + 1);
+    v = make_float4(a.z, a.w, b.x, a.x);
+  }
+  if (x > 0) {
+    const float4 a = __ldg(p + 2 * point - 2), b = __ldg(p + 2 * point - 1);
+    v.x += b.y;
+    v.y += b.z;
+    v.z += b.w;
+    v.w += a.y;
+  }
+  return v;
+}
+
 // kBlocks: resident warps per SM / 8 the register allocation is sized for.
-template <int P, int kBlocks>
+template <int P, int kBlocks, bool kEdges>
 __global__ void __launch_bounds__(kMarchThreads, 2 * kBlocks) volume_backward_kernel(VolumeArgs a) {
   const uint32_t n_subs = tile_ids(a) * (32u / a.lanes);
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -191,13 +250,13 @@ __global__ void __launch_bounds__(kMarchThreads, 2 * kBlocks) volume_backward_ke
     const float4 o4 = reinterpret_cast<const float4*>(a.rgba_fwd)[off];
     float o[3], d[3];
     pixel_ray(a.cam[cam], x, y, o, d);
-    GradVis gv;
+    GradVis<kEdges> gv;
     gv.a = &a;
     gv.g[0] = g4.x; gv.g[1] = g4.y; gv.g[2] = g4.z; gv.g[3] = g4.w;
     gv.gout = ffma(g4.w, o4.w, ffma(g4.z, o4.z, ffma(g4.y, o4.y, fmul(g4.x, o4.x))));
     gv.init();
     RayOut r;
-    march<P, GradVis, false>(a.v, o, d, gv, r);
+    march<P, GradVis<kEdges>, false>(a.v, o, d, gv, r);
     gv.flush();
     bad |= r.bad;
   }
@@ -321,12 +380,12 @@ void launch_forward(const VolumeArgs& a, uint32_t blocks, cudaStream_t s) {
     launch_march<volume_forward_kernel<P, kMinBlocks, kSkip>>(a, blocks, s);
 }
 
-template <int P>
+template <int P, bool kEdges>
 void launch_backward(const VolumeArgs& a, uint32_t blocks, cudaStream_t s) {
   if (fits_small(blocks))
-    launch_march<volume_backward_kernel<P, kSmallMinBlocks>>(a, blocks, s);
+    launch_march<volume_backward_kernel<P, kSmallMinBlocks, kEdges>>(a, blocks, s);
   else
-    launch_march<volume_backward_kernel<P, kMinBlocks>>(a, blocks, s);
+    launch_march<volume_backward_kernel<P, kMinBlocks, kEdges>>(a, blocks, s);
 }
 
 }  // namespace
@@ -373,16 +432,22 @@ cudaError_t launch_volume_forward(VolumeArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_volume_backward(VolumeArgs& a, cudaStream_t s) {
+bool backward_uses_edges(VolumeArgs& a) {
+  const uint32_t tiles = tile_ids(a);
+  set_lanes(a, tiles);
+  return !fits_small(march_blocks(a, tiles));
+}
+
+cudaError_t launch_volume_backward(VolumeArgs& a, bool edges, cudaStream_t s) {
   const uint32_t tiles = tile_ids(a);
   if (tiles == 0) return cudaSuccess;
   set_lanes(a, tiles);
   const uint32_t blocks = march_blocks(a, tiles);
   // only fp32 (learnable) volumes have an adjoint
   if (a.v.precision == 1)
-    launch_backward<1>(a, blocks, s);
+    edges ? launch_backward<1, true>(a, blocks, s) : launch_backward<1, false>(a, blocks, s);
   else if (a.v.precision == 2)
-    launch_backward<2>(a, blocks, s);
+    edges ? launch_backward<2, true>(a, blocks, s) : launch_backward<2, false>(a, blocks, s);
   else
     return cudaErrorInvalidValue;
   return cudaGetLastError();
@@ -418,10 +483,11 @@ cudaError_t launch_apron_fold(const VolumeArgs& a, int channels, float* g, bool 
   return cudaGetLastError();
 }
 
+template <bool kEdges>
 __global__ void unpack_grads_kernel(const float4* __restrict__ p, uint32_t n, float* gd,
                                     float* ga) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float4 v = p[i];
+    const float4 v = point_grad<kEdges>(p, i, (int)(i % (uint32_t)kL3 % (uint32_t)kL));
     gd[i] += v.w;
     ga[3 * (size_t)i] += v.x;
     ga[3 * (size_t)i + 1] += v.y;
@@ -429,11 +495,11 @@ __global__ void unpack_grads_kernel(const float4* __restrict__ p, uint32_t n, fl
   }
 }
 
-cudaError_t launch_unpack_grads(const float4* packed, uint32_t n, float* grad_density,
-                                float* grad_albedo, cudaStream_t s) {
+cudaError_t launch_unpack_grads(const float4* scratch, bool edges, uint32_t n,
+                                float* grad_density, float* grad_albedo, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  unpack_grads_kernel<<<2 * device_sm_count_vol() * 8, 256, 0, s>>>(packed, n, grad_density,
-                                                                     grad_albedo);
+  auto kern = edges ? unpack_grads_kernel<true> : unpack_grads_kernel<false>;
+  kern<<<2 * device_sm_count_vol() * 8, 256, 0, s>>>(scratch, n, grad_density, grad_albedo);
   return cudaGetLastError();
 }
 
@@ -506,18 +572,19 @@ cudaError_t launch_pack_train(const float* density, const float* albedo, uint32_
   return cudaGetLastError();
 }
 
-// Unpack and apron fold in one pass over the lattice points (3072 bricks: 12
-// us, where an unpack, two gathers, two scatters and the zeroing of two
+// Unpack and apron fold in one pass over the lattice points (3072 bricks: 14
+// us, 27 from edge records, where an unpack, two gathers, two scatters and the zeroing of two
 // tensors took 105): a point's owner
 // (its own brick, or the upper neighbour for an apron point) sums its copies
 // in the order of fold_gather_kernel.  Interior points have one copy and need
 // no neighbour.
-__global__ void __launch_bounds__(256) fold_packed_kernel(const float4* __restrict__ p,
-                                                          const int32_t* __restrict__ up,
-                                                          const int32_t* __restrict__ dn,
-                                                          uint32_t npoints,
-                                                          float* __restrict__ gd,
-                                                          float* __restrict__ ga) {
+template <bool kEdges>
+__global__ void __launch_bounds__(256) fold_grads_kernel(const float4* __restrict__ p,
+                                                         const int32_t* __restrict__ up,
+                                                         const int32_t* __restrict__ dn,
+                                                         uint32_t npoints,
+                                                         float* __restrict__ gd,
+                                                         float* __restrict__ ga) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < npoints;
        i += gridDim.x * blockDim.x) {
     const uint32_t b = i / (uint32_t)kL3, q = i % (uint32_t)kL3;
@@ -532,15 +599,18 @@ __global__ void __launch_bounds__(256) fold_packed_kernel(const float4* __restri
     }
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (own >= 0) {
-      v = __ldg(p + (size_t)own * kL3 + (size_t)((z * kL + y) * kL + x));
+      v = point_grad<kEdges>(p, (size_t)own * kL3 + (size_t)((z * kL + y) * kL + x), x);
       if (x == 0 || y == 0 || z == 0) {
         for (int m = 1; m < 8; ++m) {
           const int dx = m & 1, dy = (m >> 1) & 1, dz = m >> 2;
           if ((dx && x) || (dy && y) || (dz && z)) continue;
           const int nb = __ldg(dn + (size_t)own * 7 + (m - 1));
           if (nb < 0) continue;
-          const float4 c = __ldg(p + (size_t)nb * kL3 +
-                                 (size_t)(((z + 8 * dz) * kL + (y + 8 * dy)) * kL + (x + 8 * dx)));
+          const float4 c = point_grad<kEdges>(
+              p,
+              (size_t)nb * kL3 +
+                  (size_t)(((z + 8 * dz) * kL + (y + 8 * dy)) * kL + (x + 8 * dx)),
+              x + 8 * dx);
           v.x += c.x;
           v.y += c.y;
           v.z += c.z;
@@ -555,13 +625,14 @@ __global__ void __launch_bounds__(256) fold_packed_kernel(const float4* __restri
   }
 }
 
-cudaError_t launch_fold_packed(const VolumeArgs& a, const float4* packed, float* grad_density,
-                               float* grad_albedo, cudaStream_t s) {
+cudaError_t launch_fold_grads(const VolumeArgs& a, const float4* scratch, bool edges,
+                              float* grad_density, float* grad_albedo, cudaStream_t s) {
   const uint32_t n = a.v.nbricks * (uint32_t)kL3;
   if (n == 0) return cudaSuccess;
   const uint32_t blocks = (n + 255u) / 256u, cap = (uint32_t)device_sm_count_vol() * 32u;
-  fold_packed_kernel<<<blocks < cap ? blocks : cap, 256, 0, s>>>(packed, a.nbr_up, a.nbr_dn, n,
-                                                                grad_density, grad_albedo);
+  auto kern = edges ? fold_grads_kernel<true> : fold_grads_kernel<false>;
+  kern<<<blocks < cap ? blocks : cap, 256, 0, s>>>(scratch, a.nbr_up, a.nbr_dn, n, grad_density,
+                                                  grad_albedo);
   return cudaGetLastError();
 }
 

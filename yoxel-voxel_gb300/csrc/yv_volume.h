@@ -55,7 +55,8 @@ struct VolumeArgs {
   uint32_t* bricks_entered;
   const float* rgba_fwd;  // backward: forward output
   const float* grad_rgba; // backward: dL/d rgba
-  float4* grad_packed;    // backward output: (albedo rgb, density) per lattice point
+  float4* grad_scratch;   // backward output: one float4 per lattice point, two with edges
+                          // (GradVis)
   uint32_t* status;       // optional device status word
   // forward only: warp tiles [tile_begin, tile_end) of the launch (march
   // order, see tile_ids); tile_end = 0: all of them
@@ -70,7 +71,10 @@ cudaError_t launch_volume_forward(VolumeArgs& a, cudaStream_t s);
 // Warp tiles of one camera's width x height frame in the march's order:
 // 16x16-pixel squares (row-major) of 8 tiles of 8x4 pixels.
 uint32_t volume_tiles_per_camera(int width, int height);
-cudaError_t launch_volume_backward(VolumeArgs& a, cudaStream_t s);
+// Whether a backward whose largest launch is a's keeps edge records (two float4
+// per lattice point) in its gradient scratch.
+bool backward_uses_edges(VolumeArgs& a);
+cudaError_t launch_volume_backward(VolumeArgs& a, bool edges, cudaStream_t s);
 // packed[i] = (albedo rgb, density) of n lattice points (fp32 layouts).
 cudaError_t launch_pack_f32(const float* density, const float* albedo, uint32_t n,
                             float4* packed, cudaStream_t s);
@@ -78,14 +82,14 @@ cudaError_t launch_pack_f32(const float* density, const float* albedo, uint32_t 
 // the packed pool (16 words per brick) and its marked cells per brick.
 cudaError_t launch_pack_train(const float* density, const float* albedo, uint32_t nbricks,
                               float4* packed, uint32_t* mask, uint32_t* marked, cudaStream_t s);
-// grad_density / grad_albedo = the packed gradients of a.v's pool, every copy
-// of a lattice point holding the sum over its copies (0 where its owner brick
-// is absent).
-cudaError_t launch_fold_packed(const VolumeArgs& a, const float4* packed, float* grad_density,
-                               float* grad_albedo, cudaStream_t s);
-// grad_density += packed.w, grad_albedo += packed.xyz (n lattice points).
-cudaError_t launch_unpack_grads(const float4* packed, uint32_t n, float* grad_density,
-                                float* grad_albedo, cudaStream_t s);
+// grad_density / grad_albedo = the gradients in the scratch of a.v's pool, every
+// copy of a lattice point holding the sum over its copies (0 where its owner
+// brick is absent).
+cudaError_t launch_fold_grads(const VolumeArgs& a, const float4* scratch, bool edges,
+                              float* grad_density, float* grad_albedo, cudaStream_t s);
+// grad_density, grad_albedo += the gradients in the scratch (n lattice points).
+cudaError_t launch_unpack_grads(const float4* scratch, bool edges, uint32_t n,
+                                float* grad_density, float* grad_albedo, cudaStream_t s);
 // gather=true: fold apron gradients into owners, then copy owners to aprons;
 // gather=false: copy owners to aprons only (parameter sync).
 cudaError_t launch_apron_fold(const VolumeArgs& a, int channels, float* g, bool gather,
