@@ -100,10 +100,10 @@ __device__ __forceinline__ uint32_t ffc(Box& t) {
 // argmin tie order of :75-78) as the child bit it flips, and the move into
 // the sibling across it.
 __device__ __forceinline__ uint32_t exit_bit(const Box& t) {
-  const bool p = t.x2 > t.y2;
-  const bool ey = p && t.y2 < t.z2;
-  const bool ex = !p && t.x2 < t.z2;
-  return ey ? 8u : (ex ? 4u : 16u);
+  // z where z2 <= min(x2, y2), else x where x2 <= y2: the minimum, which the
+  // step needs anyway, in place of three chained compares (523 -> 514 us)
+  const float m = fmin3(t.x2, t.y2, t.z2);
+  return t.z2 == m ? 16u : (t.x2 == m ? 4u : 8u);
 }
 
 // On the crossed axis t1, t2 <- t2, t2 + (t2 - t1); predicated, the lanes of
