@@ -188,8 +188,13 @@ cudaError_t launch_batch(const BatchLaunch& b, const LaunchCfg& cfg, cudaStream_
   if (b.nitems <= 0) return cudaSuccess;
   int bt = cfg.block_threads;
   if (bt < 32 || bt > 256 || (bt & 31)) bt = 256;
-  // register budget per blocks_per_sm: 2 (default), 3, 4
-  const int mb = cfg.blocks_per_sm <= 0 ? 2 : (cfg.blocks_per_sm > 4 ? 4 : cfg.blocks_per_sm);
+  // register budget per blocks_per_sm: 2, 3, 4.  0 = by the batch's size: 3
+  // from 40 8x4-pixel tiles on per warp resident at 2, where throughput decides
+  // (16..24 scenes of 113 k..343 k tiles 1.03..1.10x faster than at 2), else 2,
+  // where each warp is faster (24 k..95 k tiles 1.03..1.15x)
+  int mb = cfg.blocks_per_sm > 4 ? 4 : cfg.blocks_per_sm;
+  if (mb <= 0)
+    mb = (uint64_t)b.total_ids / 32u >= 40ull * 16u * (uint64_t)device_sm_count() ? 3 : 2;
   switch (b.brick_precision) {
     case 0: return launch_by_budget<0>(b, mb, bt, s);
     case 1: return launch_by_budget<1>(b, mb, bt, s);
