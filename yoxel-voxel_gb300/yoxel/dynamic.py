@@ -5,11 +5,14 @@ qtview.py:69-73) over the C ABI.  Frames are traced from the device mirror
 by the caller-layout kernel (yv_render_svo_noalloc), so hit ids are the
 pool's own node ids."""
 import ctypes as C
+import struct
 
 import numpy as np
 
 from . import _lib as L
 from .svo import ATTR_DTYPE, NODE_DTYPE
+
+_pack_attr = struct.Struct("4B4b").pack  # a leaf attribute of plain integers
 
 
 def _stream(stream):
@@ -38,10 +41,13 @@ class DynamicSVO:
         """Sets the voxel to a leaf of colour rgb (None: clears it)."""
         a = None
         if rgb is not None:
-            at = np.zeros(1, ATTR_DTYPE)
-            at["rgb"][0] = [rgb[0], rgb[1], rgb[2], 255]
-            at["n"][0] = [normal[0], normal[1], normal[2], 0]
-            a = at.ctypes.data
+            try:
+                a = _pack_attr(rgb[0], rgb[1], rgb[2], 255, normal[0], normal[1], normal[2], 0)
+            except struct.error:  # not integers in range: as numpy takes or refuses them
+                at = np.zeros(1, ATTR_DTYPE)
+                at["rgb"][0] = [rgb[0], rgb[1], rgb[2], 255]
+                at["n"][0] = [normal[0], normal[1], normal[2], 0]
+                a = at.ctypes.data
         L.check(L.lib.yv_svo_dynamic_set_voxel(self._h, depth, x, y, z, a),
                 "yv_svo_dynamic_set_voxel")
 
