@@ -82,14 +82,15 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 __device__ __forceinline__ uint32_t ffc(Box& t) {
   const float te = fmax3(t.x1, t.y1, t.z1);
   uint32_t ch;
-  asm("{\n\t.reg .pred px, py, pz;\n\t.reg .f32 mx, my, mz;\n\t"
+  // te > 0.5 (x1 + x2) as 2 te > x1 + x2 (both scalings by two are exact), so
+  // that the halving is the predicated write itself
+  asm("{\n\t.reg .pred px, py, pz;\n\t.reg .f32 mx, my, mz, t2;\n\t"
       "add.rn.f32 mx, %1, %4;\n\tadd.rn.f32 my, %2, %5;\n\tadd.rn.f32 mz, %3, %6;\n\t"
-      "mul.rn.f32 mx, mx, 0f3F000000;\n\tmul.rn.f32 my, my, 0f3F000000;\n\t"
-      "mul.rn.f32 mz, mz, 0f3F000000;\n\t"
-      "setp.gt.f32 px, %7, mx;\n\tsetp.gt.f32 py, %7, my;\n\tsetp.gt.f32 pz, %7, mz;\n\t"
-      "@px mov.f32 %1, mx;\n\t@!px mov.f32 %4, mx;\n\t"
-      "@py mov.f32 %2, my;\n\t@!py mov.f32 %5, my;\n\t"
-      "@pz mov.f32 %3, mz;\n\t@!pz mov.f32 %6, mz;\n\t"
+      "add.rn.f32 t2, %7, %7;\n\t"
+      "setp.gt.f32 px, t2, mx;\n\tsetp.gt.f32 py, t2, my;\n\tsetp.gt.f32 pz, t2, mz;\n\t"
+      "@px mul.rn.f32 %1, mx, 0f3F000000;\n\t@!px mul.rn.f32 %4, mx, 0f3F000000;\n\t"
+      "@py mul.rn.f32 %2, my, 0f3F000000;\n\t@!py mul.rn.f32 %5, my, 0f3F000000;\n\t"
+      "@pz mul.rn.f32 %3, mz, 0f3F000000;\n\t@!pz mul.rn.f32 %6, mz, 0f3F000000;\n\t"
       "selp.u32 %0, 4, 0, px;\n\t@py or.b32 %0, %0, 8;\n\t@pz or.b32 %0, %0, 16;\n\t}"
       : "=&r"(ch), "+f"(t.x1), "+f"(t.y1), "+f"(t.z1), "+f"(t.x2), "+f"(t.y2), "+f"(t.z2)
       : "f"(te));
@@ -294,7 +295,7 @@ __device__ __forceinline__ Probe probe_child(const SvoDeviceScene& sc, const Tra
   } else {
     p.w = tr.codes << c;
     p.leaf = p.w >= (YV_CODE_LEAF << 28);
-    p.take = p.leaf ? (!cull || ahead) : ((int32_t)p.w >= 0 && ahead);
+    p.take = (ahead || (p.leaf && !cull)) && (p.leaf || (int32_t)p.w >= 0);
   }
   return p;
 }
