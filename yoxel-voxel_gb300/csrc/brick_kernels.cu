@@ -518,8 +518,9 @@ cudaError_t launch_pack_f32(const float* density, const float* albedo, uint32_t 
 
 // One warp per brick (blocks of 256): its 729 lattice points packed, and the
 // cell occupancy mask gathered from ballots on the way.  A point whose albedo
-// is not finite counts as set, so a sample the mask lets the march pass over
-// adds exactly nothing (0 x albedo).
+// is not finite, or so large that interpolation could overflow, counts as set,
+// so a sample the mask lets the march pass over adds exactly nothing (0 x
+// albedo).
 __global__ void __launch_bounds__(256) pack_train_kernel(const float* __restrict__ d,
                                                          const float* __restrict__ c,
                                                          uint32_t nbricks,
@@ -547,9 +548,8 @@ __global__ void __launch_bounds__(256) pack_train_kernel(const float* __restrict
       for (uint32_t u = 0; u < 8u; ++u) {
         const uint32_t k = lane + 32u * (q0 + u);
         if (k < (uint32_t)kL3) out[base + k] = v[u];
-        const bool set = v[u].w != 0.f || !(fabsf(v[u].x) <= 3.402823466e38f) ||
-                         !(fabsf(v[u].y) <= 3.402823466e38f) ||
-                         !(fabsf(v[u].z) <= 3.402823466e38f);
+        const bool set = v[u].w != 0.f || !(fabsf(v[u].x) <= 1e38f) ||
+                         !(fabsf(v[u].y) <= 1e38f) || !(fabsf(v[u].z) <= 1e38f);
         const uint32_t bits = __ballot_sync(0xFFFFFFFFu, set);
         if (lane == 0) nz[q0 + u] = bits;
       }
