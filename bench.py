@@ -231,7 +231,7 @@ def profile_l2(name):
     m = re.search(r"l2_pct_of_peak:\s*([0-9.]+)", txt)
     if m:
         out["pct_of_peak_sector_rate"] = float(m.group(1))
-    out["source"] = f"ncu --set full capture (lts__t_sectors.sum x 32 B), profiles/{name}.md"
+    out["source"] = f"ncu capture (lts__t_sectors.sum x 32 B), profiles/{name}.md"
     return out
 
 
@@ -254,7 +254,7 @@ def profile_issue(name):
         out["thread_instructions_per_unit"] = float(m.group(1))
         out["unit"] = m.group(2)
     if out:
-        out["source"] = f"ncu --set full capture, profiles/{name}.md"
+        out["source"] = f"ncu capture, profiles/{name}.md"
     return out or None
 
 
@@ -865,17 +865,18 @@ def run_train(args, cfg):
                                        "dram__bytes_write.sum), profiles/volume_backward_cfg4.md",
                      "kernel": "volume_backward_kernel", "algorithmic_bytes_per_launch": alg_b,
                      "note": "the replay reads and the gradient atomics are served by L1/L2 "
-                             "(the 29 MB gradient scratch stays in L2), so the algorithmic "
+                             "(the 59 MB gradient scratch stays in L2), so the algorithmic "
                              "bytes exceed what HBM could move in the time (frac > 1) while "
-                             "DRAM moves only `traffic`: the kernel is bound by load latency "
-                             "and L2 atomic requests, not HBM",
+                             "DRAM moves only `traffic`: the kernel is bound by the L1 "
+                             "data pipe and load latency, not HBM",
                      "issue": profile_issue("volume_backward_cfg4"),
                      "l2": profile_l2("volume_backward_cfg4")},
         "gradient_check": "GPU adjoint vs FP64 adjoint / naive PyTorch marcher / FP64 central "
                           "differences: rel. error <= 1e-4 (tests/test_volume_gpu.py)",
-        # per fwd+bwd step: pack, forward, adjoint, unpack, 2 x (fold gather +
-        # scatter); the loss and its gradient are torch's own kernels
-        "gpu_launches": args.steps * (6 + 2 * -(-ncam // 64)),
+        # per fwd+bwd step: pack (with the cell mask), forward and adjoint per
+        # 64 cameras, unpack + apron fold; the loss and its gradient are
+        # torch's own kernels
+        "gpu_launches": args.steps * (2 + 2 * -(-ncam // 64)),
         "clocks": clocks, "wall_s_timed_region": round(wall, 4)})
     host = torch.empty((), dtype=torch.float32, pin_memory=True)
     torch.cuda.synchronize()
@@ -1092,8 +1093,8 @@ def run_build(args, cfg):
                 "h2d_bytes_per_step": 4 * vox, "d2h_bytes_per_step": 40 * nn + 8 * na,
                 "path": "density from pinned host memory, yoxel.SVOScene.build_dense (pool "
                         "copied back into a host container)"},
-        # 67 kernels per 1024^3 build (the ncu launch list of the same command)
-        "gpu_launches": args.steps * 67,
+        # 11 kernels per 1024^3 build (the ncu launch list of the same command)
+        "gpu_launches": args.steps * 11,
         "gpu_launches_source": "ncu launch list, profiles/svo_build_dense_1024.md",
         "clocks": clocks, "wall_s_timed_region": round(wall, 4)})
     if not args.no_cpu_baseline:
@@ -1186,8 +1187,8 @@ def run_vbuild(args, cfg):
                 "h2d_bytes_per_step": 4 * vox, "d2h_bytes_per_step": 4 * 729 * nb * 4,
                 "path": "lattice from pinned host memory, yoxel.BrickVolume.build_dense (pool "
                         "copied back into a host container)"},
-        # 21 kernels per 513^3 rebuild (the ncu launch list of the same command)
-        "gpu_launches": args.steps * 21,
+        # 9 kernels per 513^3 rebuild (the ncu launch list of the same command)
+        "gpu_launches": args.steps * 9,
         "gpu_launches_source": "ncu launch list, profiles/volume_build_dense_513.md",
         "clocks": clocks, "wall_s_timed_region": round(wall, 4)})
     if not args.no_cpu_baseline:
@@ -1338,9 +1339,11 @@ def run_ssna(args, cfg):
     mean_trace = sum(ms_trace) / len(ms_trace)
     post_ms = max(mean - mean_trace, 1e-6)
     # algorithmic bytes of the post chain per pixel: depth (albedo + t in, z
-    # out: 12), each blur pass (z in + out: 8), shading (albedo, z, stored
-    # normal in, rgba out: 24)
-    post_bytes = npix * (12 + 8 * cfg["passes"] + 24)
+    # out: 12), each blur pass launched (z in + out: 8), shading (albedo, z,
+    # stored normal in, rgba out: 24); the limits of 2 passes reach the scene
+    # (the ncu launch list of the same command)
+    blurs = min(2, cfg["passes"])
+    post_bytes = npix * (12 + 8 * blurs + 24)
     peaks, peak_kind = measured_peaks()
     achieved = post_bytes / (post_ms / 1e3) / 1e9
 
@@ -1372,7 +1375,9 @@ def run_ssna(args, cfg):
                 "h2d_bytes_per_step": C.sizeof(L.SsnaParams),
                 "d2h_bytes_per_step": npix * 4,
                 "path": "yv_render_ssna (C ABI) + frame copy into pinned host memory"},
-        "gpu_launches": (int(st["launches"]) + 2 + cfg["passes"]) * args.steps,
+        # trace, depth, blur passes and shading
+        "gpu_launches": (int(st["launches"]) + 2 + blurs) * args.steps,
+        "gpu_launches_source": "ncu launch list, profiles/ssna_post_chain_1080p.md",
         "clocks": clocks})
     if not args.no_cpu_baseline:
         from oracle import ssna as O
