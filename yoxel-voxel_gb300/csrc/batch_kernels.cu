@@ -103,11 +103,12 @@ __global__ void __launch_bounds__(256, kMinBlocks) batch_kernel(BatchLaunch b) {
       continue;
     }
 
-    // up to kStepsPerVote traversal steps, then the end of a ray once
+    // up to kStepsPerVote traversal steps, then the end of a ray once (16
+    // scenes 1762 us whatever their number; 1854 with 24 copies of the step)
     const BatchItem& it = items[item];
     int r = kContinue;
     uint32_t leaf = 0;
-#pragma unroll
+#pragma unroll 4
     for (int k = 0; k < kStepsPerVote; ++k)
       if ((mode == kPrimary || mode == kShadow) && r == kContinue)
         r = trace_step<false, kBatchRing>(it.svo, nullptr, 0u, stk, ring, tr, mode == kShadow,

@@ -49,10 +49,13 @@ namespace yv {
 namespace {
 
 constexpr uint32_t kFetchCap = 1u << 20;
-// traversal steps between two warp votes (refill / end-of-ray handling); 12
-// measured slower (576 against 524 us on a 1920x1080 frame with shadow rays).
-// Unrolled 4 deep: 8 copies of the step overflow the instruction cache.
-constexpr int kStepsPerVote = 8;
+// Traversal steps between two warp votes (refill / end-of-ray handling): a vote
+// and a pass through the end of a ray cost every lane of the warp, a lane whose
+// ray has ended waits for the rest of its group.  1920x1080 frame with shadow
+// rays / 160x120 / 641x479 with the detail cut-off: 512 / 50.5 / 96.5 us at 8
+// steps, 502 / 49.3 / 93.7 at 24, 512 / 49.3 / 93.8 at 48.  Unrolled 6 deep
+// (504 us at 4): more copies overflow the instruction cache.
+constexpr int kStepsPerVote = 24;
 
 struct Box {
   float x1, y1, z1, x2, y2, z2;
@@ -594,7 +597,7 @@ __global__ void __launch_bounds__(256, kMinBlocks)
     for (;;) {
       int r = kContinue;
       uint32_t leaf = 0;
-#pragma unroll 4
+#pragma unroll 6
       for (int k = 0; k < kStepsPerVote; ++k)
         if ((mode == kPrimary || mode == kShadow) && r == kContinue)
           r = trace_step<kRef, kRing, kStaged, kLod>(sc, smw, nsm, stk, ring, tr,
