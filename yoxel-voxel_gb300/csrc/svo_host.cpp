@@ -1001,53 +1001,59 @@ yv_status build_device_layout(const yv_vox_node* nodes, uint32_t count,
   }
   out->depth = height[root];
   // breadth-first records: the run of a node's children is laid down when its
-  // first record is reached (run[id]), and shared by its other records
-  std::vector<uint32_t> run(count, 0xFFFFFFFFu), leaves(count, 0);
+  // first record (first[id]) is reached, and shared by its other records.  The
+  // table of the leaves' attributes is kept from the first leaf on that is not
+  // numbered as its attribute.
+  std::vector<uint32_t> first(count, 0xFFFFFFFFu);
   std::vector<uint32_t> order;  // record -> caller node id
+  order.reserve(count);
   order.push_back(root);
+  out->nodes.reserve(2 * (size_t)count);
+  out->cold.reserve(2 * (size_t)count);
   uint64_t n_leaves = 0;
+  bool same = true;
   for (size_t i = 0; i < order.size(); ++i) {
     const uint32_t id = order[i];
-    if (run[id] != 0xFFFFFFFFu) continue;
-    const yv_vox_node& n = nodes[id];
-    run[id] = (uint32_t)order.size();
-    leaves[id] = (uint32_t)n_leaves;
+    if (first[id] != 0xFFFFFFFFu) {
+      const size_t f = first[id];
+      const uint32_t run = out->nodes[2 * f], codes = out->nodes[2 * f + 1],
+                     leaf = out->cold[2 * f + 1];
+      out->nodes.push_back(run);
+      out->nodes.push_back(codes);
+      out->cold.push_back(id);
+      out->cold.push_back(leaf);
+      continue;
+    }
+    first[id] = (uint32_t)i;
     ++out->n_unique;
+    const yv_vox_node& n = nodes[id];
+    uint32_t codes = 0, rank = 0;
+    out->nodes.push_back((uint32_t)order.size());
+    out->cold.push_back(id);
+    out->cold.push_back((uint32_t)n_leaves);
     for (int ch = 0; ch < 8; ++ch) {
       const uint32_t w = n.child[ch];
+      uint32_t k = YV_CODE_NULL;
       if ((n.flags >> ch) & 1u) {
-        out->leaf_attr.push_back(w);
+        k = YV_CODE_LEAF;
+        if (same && w != n_leaves) {
+          same = false;
+          out->leaf_attr.resize((size_t)n_leaves);
+          for (size_t l = 0; l < out->leaf_attr.size(); ++l) out->leaf_attr[l] = (uint32_t)l;
+        }
+        if (!same) out->leaf_attr.push_back(w);
         ++n_leaves;
       } else if (!(w & 0x80000000u)) {
+        k = rank++;
         order.push_back(w);
       }
+      codes |= k << (28 - 4 * ch);
     }
+    out->nodes.push_back(codes);
     if (order.size() > YV_MAX_DEVICE_NODES || n_leaves > 0xFFFFFFFEull) {
       *why = "pool larger than 2^29 nodes";
       return YV_ERR_BAD_POOL;
     }
-  }
-  bool same = true;  // leaves already numbered as their attributes
-  for (size_t i = 0; i < out->leaf_attr.size() && same; ++i) same = out->leaf_attr[i] == i;
-  if (same) out->leaf_attr.clear();
-  out->nodes.resize(order.size() * 2);
-  out->cold.resize(order.size() * 2);
-  for (size_t i = 0; i < order.size(); ++i) {
-    const uint32_t id = order[i];
-    const yv_vox_node& n = nodes[id];
-    uint32_t codes = 0, rank = 0;
-    for (int ch = 0; ch < 8; ++ch) {
-      uint32_t k = YV_CODE_NULL;
-      if ((n.flags >> ch) & 1u)
-        k = YV_CODE_LEAF;
-      else if (!(n.child[ch] & 0x80000000u))
-        k = rank++;
-      codes |= k << (28 - 4 * ch);
-    }
-    out->nodes[2 * i] = run[id];
-    out->nodes[2 * i + 1] = codes;
-    out->cold[2 * i] = id;
-    out->cold[2 * i + 1] = leaves[id];
   }
   out->root_word = 0;
   return YV_OK;
