@@ -97,10 +97,11 @@ __global__ void solid_bits_kernel(Grid g, uint32_t WR, uint32_t* S) {
   }
 }
 
-// Pass 1a for rows of 128 voxels or more (G >= 128): one 128-voxel chunk
-// per warp and iteration, each lane a 16-byte load of 4 voxels; the lanes'
-// 4-bit groups are ORed into 32-bit words within groups of 8 lanes (3
-// shuffles), lane 8j writing word j of the chunk.  Same bits as above.
+// Pass 1a for rows of 128 voxels or more (G >= 128) of a grid that starts on
+// a 16-byte boundary: one 128-voxel chunk per warp and iteration, each lane a
+// 16-byte load of 4 voxels; the lanes' 4-bit groups are ORed into 32-bit words
+// within groups of 8 lanes (3 shuffles), lane 8j writing word j of the chunk.
+// Same bits as above.
 __global__ void solid_bits_v4_kernel(Grid g, uint32_t WR, uint32_t* S) {
   constexpr int kU = 4;
   const uint32_t lane = threadIdx.x & 31u;
@@ -700,7 +701,8 @@ yv_status count_dense(const float* density, const uint8_t* rgb, int depth, float
   if ((e = cudaMemsetAsync(b.node, 0, head, s)) != cudaSuccess ||
       (e = cudaMemsetAsync(b.full, 0, head, s)) != cudaSuccess)
     return build_fail(e, "clear");
-  if (G >= 128)
+  // (a view into a larger array need not be aligned for the 16-byte loads)
+  if (G >= 128 && (reinterpret_cast<uintptr_t>(density) & 15u) == 0)
     solid_bits_v4_kernel<<<grid_for((uint64_t)G * G * b.WR * 8), 256, 0, s>>>(b.g, b.WR, b.S);
   else
     solid_bits_kernel<<<grid_for((uint64_t)G * G * b.WR * 32 / 4), 256, 0, s>>>(b.g, b.WR, b.S);
