@@ -379,7 +379,8 @@ typedef struct yv_volume_device {
   int32_t levels;
   const void* density;
   const void* albedo;
-  uint32_t nbricks;
+  uint32_t nbricks;     /* up to 2^32 / 729: lattice points have 32-bit numbers
+                         * (more: YV_ERR_UNSUPPORTED) */
   int32_t precision;
   const int32_t* nbr_up;
   const int32_t* nbr_dn;

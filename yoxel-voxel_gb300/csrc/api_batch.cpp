@@ -210,6 +210,8 @@ yv_status yv_batch_add_volume(yv_batch* b, const yv_volume_device* vol, const yv
       (vol->nbricks && vol->precision < YV_PRECISION_F32_PACKED && !vol->density))
     return YV_ERR_INVALID_ARG;
   if ((int)b->items.size() >= kMaxBatchItems) return YV_ERR_UNSUPPORTED;
+  const yv_status fits = pool_points_fit(vol->nbricks);
+  if (fits != YV_OK) return fits;
   BatchItem it{};
   it.kind = kBatchBrick;
   it.width = width;

@@ -121,9 +121,23 @@ bool cams_ok(const yv_camera* c, int n) {
   return true;
 }
 
+// The arguments of a call that reads the lattice points of the pool.
+yv_status march_args(const yv_volume_device* v, const yv_march_params* mp, int width, int height,
+                     VolumeArgs* a) {
+  if (!fill_args(v, mp, width, height, a)) return YV_ERR_INVALID_ARG;
+  return pool_points_fit(v->nbricks);
+}
+
 }  // namespace
 
 namespace yv {
+
+yv_status pool_points_fit(uint32_t nbricks) {
+  if (nbricks <= kMaxPoolBricks) return YV_OK;
+  set_last_error("brick pool of " + std::to_string(nbricks) + " bricks: at most " +
+                 std::to_string(kMaxPoolBricks) + " (2^32 lattice points)");
+  return YV_ERR_UNSUPPORTED;
+}
 
 yv_status volume_gpu_from_device(void* mem[5], const size_t bytes[5], const yv_volume_device& d,
                                  yv_volume_gpu** out, uint32_t* accel) {
@@ -236,6 +250,11 @@ yv_status yv_volume_upload(const yv_volume_host* v, int32_t precision, yv_volume
   if (!g) return YV_ERR_OUT_OF_MEMORY;
   cudaGetDevice(&g->device);
   const uint32_t ng = yv_volume_grid_count(v), nb = yv_volume_brick_count(v);
+  const yv_status fits = pool_points_fit(nb);
+  if (fits != YV_OK) {
+    delete g;
+    return fits;
+  }
   const size_t n = (size_t)nb * 729u;
   const float* den = yv_volume_density(v);
   const uint8_t* alb = yv_volume_albedo(v);
@@ -353,9 +372,11 @@ yv_status yv_volume_render(const yv_volume_device* vol, const yv_camera* cams, i
                            uint32_t* samples, uint32_t* bricks, void* stream) {
   VolumeArgs* a = new (std::nothrow) VolumeArgs;
   if (!a) return YV_ERR_OUT_OF_MEMORY;
-  if (!fill_args(vol, mp, width, height, a) || !cams_ok(cams, ncams) || !rgba) {
+  yv_status st = march_args(vol, mp, width, height, a);
+  if (st == YV_OK && (!cams_ok(cams, ncams) || !rgba)) st = YV_ERR_INVALID_ARG;
+  if (st != YV_OK) {
     delete a;
-    return YV_ERR_INVALID_ARG;
+    return st;
   }
   const size_t px = (size_t)width * (size_t)height;
   for (int c0 = 0; c0 < ncams; c0 += kMaxVolumeCams) {
@@ -388,9 +409,11 @@ yv_status yv_volume_render_tiles(const yv_volume_device* vol, const yv_camera* c
   if (ncams > kMaxVolumeCams) return YV_ERR_INVALID_ARG;
   VolumeArgs* a = new (std::nothrow) VolumeArgs;
   if (!a) return YV_ERR_OUT_OF_MEMORY;
-  if (!fill_args(vol, mp, width, height, a) || !cams_ok(cams, ncams) || !rgba) {
+  yv_status st = march_args(vol, mp, width, height, a);
+  if (st == YV_OK && (!cams_ok(cams, ncams) || !rgba)) st = YV_ERR_INVALID_ARG;
+  if (st != YV_OK) {
     delete a;
-    return YV_ERR_INVALID_ARG;
+    return st;
   }
   const uint64_t total = (uint64_t)volume_tiles_per_camera(width, height) * (uint64_t)ncams;
   if (tile_begin > tile_end || tile_end > total) {
@@ -418,9 +441,11 @@ yv_status yv_volume_render_rgba8(const yv_volume_device* vol, const yv_camera* c
                                  const yv_march_params* mp, uint32_t* rgba8, void* stream) {
   VolumeArgs* a = new (std::nothrow) VolumeArgs;
   if (!a) return YV_ERR_OUT_OF_MEMORY;
-  if (!fill_args(vol, mp, width, height, a) || !cams_ok(cams, ncams) || !rgba8) {
+  yv_status st = march_args(vol, mp, width, height, a);
+  if (st == YV_OK && (!cams_ok(cams, ncams) || !rgba8)) st = YV_ERR_INVALID_ARG;
+  if (st != YV_OK) {
     delete a;
-    return YV_ERR_INVALID_ARG;
+    return st;
   }
   const size_t px = (size_t)width * (size_t)height;
   for (int c0 = 0; c0 < ncams; c0 += kMaxVolumeCams) {
@@ -452,10 +477,14 @@ static yv_status run_backward(const yv_volume_device* vol, const yv_camera* cams
                               Finish finish) {
   VolumeArgs* a = new (std::nothrow) VolumeArgs;
   if (!a) return YV_ERR_OUT_OF_MEMORY;
-  if (!fill_args(vol, mp, width, height, a) || !cams_ok(cams, ncams) || !rgba || !grad_rgba ||
-      (vol->precision != YV_PRECISION_F32 && vol->precision != YV_PRECISION_F32_PACKED)) {
+  yv_status st = march_args(vol, mp, width, height, a);
+  if (st == YV_OK &&
+      (!cams_ok(cams, ncams) || !rgba || !grad_rgba ||
+       (vol->precision != YV_PRECISION_F32 && vol->precision != YV_PRECISION_F32_PACKED)))
+    st = YV_ERR_INVALID_ARG;
+  if (st != YV_OK) {
     delete a;
-    return YV_ERR_INVALID_ARG;
+    return st;
   }
   const size_t px = (size_t)width * (size_t)height;
   const size_t npts = (size_t)vol->nbricks * 729u;
@@ -522,9 +551,11 @@ yv_status yv_volume_train_forward(const yv_volume_device* vol, const float* dens
   d.cell_mask = d.nbricks ? mask : nullptr;
   VolumeArgs* a = new (std::nothrow) VolumeArgs;
   if (!a) return YV_ERR_OUT_OF_MEMORY;
-  if (!fill_args(&d, mp, width, height, a) || !cams_ok(cams, ncams) || !rgba) {
+  yv_status st = march_args(&d, mp, width, height, a);
+  if (st == YV_OK && (!cams_ok(cams, ncams) || !rgba)) st = YV_ERR_INVALID_ARG;
+  if (st != YV_OK) {
     delete a;
-    return YV_ERR_INVALID_ARG;
+    return st;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   uint32_t* marked = d.nbricks ? mask + (size_t)d.nbricks * 16u : nullptr;
@@ -562,7 +593,8 @@ yv_status yv_volume_fold_aprons(const yv_volume_device* vol, float* grad_density
   if (!vol || !vol->nbr_up || !vol->nbr_dn) return YV_ERR_INVALID_ARG;
   VolumeArgs a;
   yv_march_params mp = {1.f, 1.f};
-  if (!fill_args(vol, &mp, 1, 1, &a)) return YV_ERR_INVALID_ARG;
+  const yv_status st = march_args(vol, &mp, 1, 1, &a);
+  if (st != YV_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaSuccess;
   if (grad_density) e = launch_apron_fold(a, 1, grad_density, true, s);
@@ -577,7 +609,8 @@ yv_status yv_volume_sync_aprons(const yv_volume_device* vol, float* density, flo
     return YV_ERR_INVALID_ARG;
   VolumeArgs a;
   yv_march_params mp = {1.f, 1.f};
-  if (!fill_args(vol, &mp, 1, 1, &a)) return YV_ERR_INVALID_ARG;
+  const yv_status st = march_args(vol, &mp, 1, 1, &a);
+  if (st != YV_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaSuccess;
   if (density) e = launch_apron_fold(a, 1, density, false, s);

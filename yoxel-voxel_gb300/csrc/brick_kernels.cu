@@ -330,7 +330,8 @@ __global__ void fold_gather_kernel(VolumeArgs a, int channels, float* g) {
 // takes the value of the lattice point's owner, or 0 if the owner is absent.
 __global__ void fold_scatter_kernel(VolumeArgs a, int channels, float* g) {
   const uint32_t n = a.v.nbricks * (uint32_t)kL3;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (uint64_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const uint32_t i = (uint32_t)k;  // (k: n may be within a stride of 2^32)
     const uint32_t b = i / kL3, p = i % kL3;
     const int x = (int)(p % kL), y = (int)((p / kL) % kL), z = (int)(p / (kL * kL));
     const int dx = x == 8, dy = y == 8, dz = z == 8;
@@ -486,7 +487,8 @@ cudaError_t launch_apron_fold(const VolumeArgs& a, int channels, float* g, bool 
 template <bool kEdges>
 __global__ void unpack_grads_kernel(const float4* __restrict__ p, uint32_t n, float* gd,
                                     float* ga) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (uint64_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const uint32_t i = (uint32_t)k;  // (k: n may be within a stride of 2^32)
     const float4 v = point_grad<kEdges>(p, i, (int)(i % (uint32_t)kL3 % (uint32_t)kL));
     gd[i] += v.w;
     ga[3 * (size_t)i] += v.x;
@@ -505,8 +507,8 @@ cudaError_t launch_unpack_grads(const float4* scratch, bool edges, uint32_t n,
 
 __global__ void pack_f32_kernel(const float* __restrict__ d, const float* __restrict__ c,
                                 uint32_t n, float4* __restrict__ out) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    out[i] = make_float4(c[3 * (size_t)i], c[3 * (size_t)i + 1], c[3 * (size_t)i + 2], d[i]);
+  for (uint64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    out[i] = make_float4(c[3 * i], c[3 * i + 1], c[3 * i + 2], d[i]);
 }
 
 cudaError_t launch_pack_f32(const float* density, const float* albedo, uint32_t n,
@@ -585,8 +587,9 @@ __global__ void __launch_bounds__(256) fold_grads_kernel(const float4* __restric
                                                          uint32_t npoints,
                                                          float* __restrict__ gd,
                                                          float* __restrict__ ga) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < npoints;
-       i += gridDim.x * blockDim.x) {
+  for (uint64_t k = blockIdx.x * blockDim.x + threadIdx.x; k < npoints;
+       k += gridDim.x * blockDim.x) {
+    const uint32_t i = (uint32_t)k;  // (k: npoints may be within a stride of 2^32)
     const uint32_t b = i / (uint32_t)kL3, q = i % (uint32_t)kL3;
     int x = (int)(q % kL), y = (int)((q / kL) % kL), z = (int)(q / (kL * kL));
     const int m0 = (x == 8) | ((y == 8) << 1) | ((z == 8) << 2);

@@ -675,6 +675,7 @@ yv_status upload_dense(const float* density, const uint8_t* rgb, int32_t levels,
     return YV_ERR_INVALID_ARG;
   VolumeTree t;
   yv_status st = build_volume_tree(g, levels, s, t);
+  if (st == YV_OK) st = pool_points_fit(t.nbricks);
   if (st != YV_OK) return st;
   const size_t n = (size_t)t.nbricks * kVL3;
   size_t dbytes = 0, abytes = 0;

@@ -106,6 +106,13 @@ yv_status renderer_scene_buffers(yv_renderer* r, uint32_t nn, uint32_t na, uint2
                                  uint2** cold, void** attrs);
 void renderer_commit_scene(yv_renderer* r, uint32_t nn, uint32_t na, uint32_t root_word);
 
+// Bricks of the largest pool the march reads: the kernels number its lattice
+// points (729 per brick) with 32 bits.
+constexpr uint32_t kMaxPoolBricks = 0xFFFFFFFFu / 729u;
+// YV_OK, or YV_ERR_UNSUPPORTED (and its message) for a pool of more bricks than
+// kMaxPoolBricks.
+yv_status pool_points_fit(uint32_t nbricks);
+
 // A host brick volume from parts built on the device (volume_host.cpp):
 // grids (ngrids x 64 refs), fp32 lattice values and RGB per brick, brick
 // cells; the apron neighbour tables are derived here.

@@ -251,6 +251,8 @@ def pack_volume(density, albedo, out=None, stream=None):
     (nbricks, 729, 3): one 16-byte load per trilinear corner in the march."""
     torch = _torch()
     nb = density.shape[0]
+    if nb * 729 > 0xFFFFFFFF:  # (the call takes a 32-bit count)
+        raise ValueError(f"{nb} bricks: more than 2^32 lattice points")
     if out is None:
         out = torch.empty((nb, 729, 4), dtype=torch.float32, device=density.device)
     L.check(L.lib.yv_volume_pack(C.c_void_p(density.data_ptr()), C.c_void_p(albedo.data_ptr()),
