@@ -372,7 +372,11 @@ yv_status yv_volume_build_dense(const float* density, const uint8_t* rgb,
                                 int32_t levels, void* stream,
                                 yv_volume_host** out);
 
-/* Device view of a volume: all pointers are device pointers. */
+/* Device view of a volume: all pointers are device pointers.  A lattice point
+ * or a colour of the pool is read whole, so `density` and `albedo` start on a
+ * multiple of its size (F16: 2 and 4 bytes, F32: 4 and 4, F32_PACKED: albedo
+ * 16, F16_PACKED: albedo 8); other pools are YV_ERR_INVALID_ARG where they are
+ * marched. */
 typedef struct yv_volume_device {
   const uint32_t* grids;
   uint32_t ngrids;
@@ -453,8 +457,9 @@ typedef struct yv_march_params {
 
 /* Front-to-back composited RGBA (4 floats per pixel, camera-major) of
  * ncams cameras; the volume counterpart of RunTrace
- * (ntree/ntree_trace.cuh:27).  samples / bricks (optional, uint32 per
- * pixel) count samples taken and occupied bricks entered. */
+ * (ntree/ntree_trace.cuh:27).  rgba starts on a 16-byte boundary, here and
+ * in every call that reads or writes float4 frames (else
+ * YV_ERR_INVALID_ARG).  samples / bricks (optional, uint32 per pixel) count samples taken and occupied bricks entered. */
 yv_status yv_volume_render(const yv_volume_device* vol, const yv_camera* cams,
                            int32_t ncams, int32_t width, int32_t height,
                            const yv_march_params* mp, float* rgba,
@@ -478,9 +483,6 @@ yv_status yv_volume_render_tiles(const yv_volume_device* vol, const yv_camera* c
                                  uint32_t tile_end, float* rgba, uint32_t* samples,
                                  uint32_t* bricks, void* stream);
 
-/* Adjoint of yv_volume_render (fp32 volumes, plain or packed): re-marches
- * every ray and accumulates dL/ddensity and dL/dalbedo (pool layout, ADDED
- * to the buffers) from dL/drgba, given the forward output rgba. */
 /* RunTrace(const RenderParams&, uchar4* img, float*) (ntree/ntree_trace.cuh:
  * 22-28): the same march written as RGBA8 pixels, each channel
  * saturate(v) * 255 truncated, R in the low byte (float2uint,
@@ -489,6 +491,10 @@ yv_status yv_volume_render_rgba8(const yv_volume_device* vol, const yv_camera* c
                                  int32_t ncams, int32_t width, int32_t height,
                                  const yv_march_params* mp, uint32_t* rgba8,
                                  void* stream);
+/* Adjoint of yv_volume_render (fp32 volumes, plain or packed): re-marches
+ * every ray and accumulates dL/ddensity and dL/dalbedo (pool layout, ADDED
+ * to the buffers) from dL/drgba, given the forward output rgba.
+ * rgba and grad_rgba start on a 16-byte boundary. */
 yv_status yv_volume_backward(const yv_volume_device* vol,
                              const yv_camera* cams, int32_t ncams,
                              int32_t width, int32_t height,
@@ -555,7 +561,8 @@ yv_status yv_batch_add_svo(yv_batch* b, const yv_renderer* r, void* d_rgba);
  * per-scene launch does. */
 yv_status yv_batch_add_svo_outputs(yv_batch* b, const yv_renderer* r,
                                    const yv_frame_outputs* out);
-/* Adds one camera of a device volume; output: device RGBA float4. */
+/* Adds one camera of a device volume; output: device RGBA float4, 16-byte
+ * aligned. */
 yv_status yv_batch_add_volume(yv_batch* b, const yv_volume_device* vol,
                               const yv_camera* cam, int32_t width,
                               int32_t height, const yv_march_params* mp,
@@ -588,8 +595,8 @@ yv_status yv_batch_info(const yv_batch* b, uint32_t* n_items, uint64_t* rays);
  * launch errors only; malformed pools are contained by the kernel's bounds
  * checks (validate the host copy with yv_svo_validate), and the frame's
  * device status is read with yv_render_svo_noalloc_status.  Frames needing more
- * than 2^31 rays (8x4-tile padded) or pools over 2^29 nodes return
- * YV_ERR_INVALID_ARG. */
+ * than 2^31 rays (8x4-tile padded), pools over 2^29 nodes or attrs that do not
+ * start on an 8-byte boundary return YV_ERR_INVALID_ARG. */
 yv_status yv_render_svo_noalloc(const yv_vox_node* nodes, uint32_t count,
                                 uint32_t root, const yv_leaf_attr* attrs,
                                 uint32_t nattrs, const yv_camera* cam,

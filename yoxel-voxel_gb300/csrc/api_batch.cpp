@@ -207,7 +207,9 @@ yv_status yv_batch_add_volume(yv_batch* b, const yv_volume_device* vol, const yv
       vol->levels < 1 || vol->levels > 5 || !(mp->step_vox > 0.f) ||
       !(cam->fov_deg > 0.f && cam->fov_deg < 180.f) || vol->precision < YV_PRECISION_F16 ||
       vol->precision > YV_PRECISION_F16_PACKED || (vol->nbricks && !vol->albedo) ||
-      (vol->nbricks && vol->precision < YV_PRECISION_F32_PACKED && !vol->density))
+      (vol->nbricks && vol->precision < YV_PRECISION_F32_PACKED && !vol->density) ||
+      (vol->nbricks && !pool_aligned(vol->density, vol->albedo, vol->precision)) ||
+      !aligned_to(d_rgba, 16))
     return YV_ERR_INVALID_ARG;
   if ((int)b->items.size() >= kMaxBatchItems) return YV_ERR_UNSUPPORTED;
   const yv_status fits = pool_points_fit(vol->nbricks);

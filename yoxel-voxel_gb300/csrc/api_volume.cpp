@@ -124,7 +124,9 @@ bool cams_ok(const yv_camera* c, int n) {
 // The arguments of a call that reads the lattice points of the pool.
 yv_status march_args(const yv_volume_device* v, const yv_march_params* mp, int width, int height,
                      VolumeArgs* a) {
-  if (!fill_args(v, mp, width, height, a)) return YV_ERR_INVALID_ARG;
+  if (!fill_args(v, mp, width, height, a) ||
+      (v->nbricks && !pool_aligned(v->density, v->albedo, v->precision)))
+    return YV_ERR_INVALID_ARG;
   return pool_points_fit(v->nbricks);
 }
 
@@ -137,6 +139,15 @@ yv_status pool_points_fit(uint32_t nbricks) {
   set_last_error("brick pool of " + std::to_string(nbricks) + " bricks: at most " +
                  std::to_string(kMaxPoolBricks) + " (2^32 lattice points)");
   return YV_ERR_UNSUPPORTED;
+}
+
+bool pool_aligned(const void* density, const void* albedo, int precision) {
+  switch (precision) {
+    case YV_PRECISION_F16: return aligned_to(density, 2) && aligned_to(albedo, 4);
+    case YV_PRECISION_F32: return aligned_to(density, 4) && aligned_to(albedo, 4);
+    case YV_PRECISION_F32_PACKED: return aligned_to(albedo, 16);
+    default: return aligned_to(albedo, 8);
+  }
 }
 
 yv_status volume_gpu_from_device(void* mem[5], const size_t bytes[5], const yv_volume_device& d,
@@ -373,7 +384,8 @@ yv_status yv_volume_render(const yv_volume_device* vol, const yv_camera* cams, i
   VolumeArgs* a = new (std::nothrow) VolumeArgs;
   if (!a) return YV_ERR_OUT_OF_MEMORY;
   yv_status st = march_args(vol, mp, width, height, a);
-  if (st == YV_OK && (!cams_ok(cams, ncams) || !rgba)) st = YV_ERR_INVALID_ARG;
+  if (st == YV_OK && (!cams_ok(cams, ncams) || !rgba || !aligned_to(rgba, 16)))
+    st = YV_ERR_INVALID_ARG;
   if (st != YV_OK) {
     delete a;
     return st;
@@ -410,7 +422,8 @@ yv_status yv_volume_render_tiles(const yv_volume_device* vol, const yv_camera* c
   VolumeArgs* a = new (std::nothrow) VolumeArgs;
   if (!a) return YV_ERR_OUT_OF_MEMORY;
   yv_status st = march_args(vol, mp, width, height, a);
-  if (st == YV_OK && (!cams_ok(cams, ncams) || !rgba)) st = YV_ERR_INVALID_ARG;
+  if (st == YV_OK && (!cams_ok(cams, ncams) || !rgba || !aligned_to(rgba, 16)))
+    st = YV_ERR_INVALID_ARG;
   if (st != YV_OK) {
     delete a;
     return st;
@@ -479,7 +492,8 @@ static yv_status run_backward(const yv_volume_device* vol, const yv_camera* cams
   if (!a) return YV_ERR_OUT_OF_MEMORY;
   yv_status st = march_args(vol, mp, width, height, a);
   if (st == YV_OK &&
-      (!cams_ok(cams, ncams) || !rgba || !grad_rgba ||
+      (!cams_ok(cams, ncams) || !rgba || !grad_rgba || !aligned_to(rgba, 16) ||
+       !aligned_to(grad_rgba, 16) ||
        (vol->precision != YV_PRECISION_F32 && vol->precision != YV_PRECISION_F32_PACKED)))
     st = YV_ERR_INVALID_ARG;
   if (st != YV_OK) {
@@ -542,7 +556,7 @@ yv_status yv_volume_train_forward(const yv_volume_device* vol, const float* dens
                                   int32_t width, int32_t height, const yv_march_params* mp,
                                   float* packed, uint32_t* mask, float* rgba, void* stream) {
   if (!vol || (vol->nbricks && (!density || !albedo || !packed || !mask ||
-                                (reinterpret_cast<uintptr_t>(packed) & 15u))))
+                                !aligned_to(packed, 16))))
     return YV_ERR_INVALID_ARG;
   yv_volume_device d = *vol;
   d.density = nullptr;
@@ -552,7 +566,8 @@ yv_status yv_volume_train_forward(const yv_volume_device* vol, const float* dens
   VolumeArgs* a = new (std::nothrow) VolumeArgs;
   if (!a) return YV_ERR_OUT_OF_MEMORY;
   yv_status st = march_args(&d, mp, width, height, a);
-  if (st == YV_OK && (!cams_ok(cams, ncams) || !rgba)) st = YV_ERR_INVALID_ARG;
+  if (st == YV_OK && (!cams_ok(cams, ncams) || !rgba || !aligned_to(rgba, 16)))
+    st = YV_ERR_INVALID_ARG;
   if (st != YV_OK) {
     delete a;
     return st;
@@ -593,7 +608,8 @@ yv_status yv_volume_fold_aprons(const yv_volume_device* vol, float* grad_density
   if (!vol || !vol->nbr_up || !vol->nbr_dn) return YV_ERR_INVALID_ARG;
   VolumeArgs a;
   yv_march_params mp = {1.f, 1.f};
-  const yv_status st = march_args(vol, &mp, 1, 1, &a);
+  if (!fill_args(vol, &mp, 1, 1, &a)) return YV_ERR_INVALID_ARG;
+  const yv_status st = pool_points_fit(vol->nbricks);
   if (st != YV_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaSuccess;
@@ -609,7 +625,8 @@ yv_status yv_volume_sync_aprons(const yv_volume_device* vol, float* density, flo
     return YV_ERR_INVALID_ARG;
   VolumeArgs a;
   yv_march_params mp = {1.f, 1.f};
-  const yv_status st = march_args(vol, &mp, 1, 1, &a);
+  if (!fill_args(vol, &mp, 1, 1, &a)) return YV_ERR_INVALID_ARG;
+  const yv_status st = pool_points_fit(vol->nbricks);
   if (st != YV_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaSuccess;
@@ -621,7 +638,7 @@ yv_status yv_volume_sync_aprons(const yv_volume_device* vol, float* density, flo
 yv_status yv_volume_pack(const float* density, const float* albedo, uint32_t npoints,
                          float* packed, void* stream) {
   if (!npoints) return YV_OK;
-  if (!density || !albedo || !packed || (reinterpret_cast<uintptr_t>(packed) & 15u))
+  if (!density || !albedo || !packed || !aligned_to(packed, 16))
     return YV_ERR_INVALID_ARG;
   cudaError_t e = launch_pack_f32(density, albedo, npoints, reinterpret_cast<float4*>(packed),
                                   static_cast<cudaStream_t>(stream));

@@ -64,7 +64,8 @@ extern "C" yv_status yv_render_svo_noalloc(const yv_vox_node* nodes, uint32_t co
                                            int32_t height, const yv_frame_outputs* out,
                                            void* stream) {
   if (!cam || !light || !out || width <= 0 || height <= 0 ||
-      (!(root & 0x80000000u) && (!nodes || root >= count)) || (nattrs && !attrs))
+      (!(root & 0x80000000u) && (!nodes || root >= count)) || (nattrs && !attrs) ||
+      (nattrs && !aligned_to(attrs, 8)))  // (records are read whole)
     return YV_ERR_INVALID_ARG;
   if (!(cam->fov_deg > 0.f && cam->fov_deg < 180.f)) return YV_ERR_INVALID_ARG;
   // The queue counter in the scratch array indexes rays in 8x4 tiles; a

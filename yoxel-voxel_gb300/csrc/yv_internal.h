@@ -112,6 +112,13 @@ constexpr uint32_t kMaxPoolBricks = 0xFFFFFFFFu / 729u;
 // YV_OK, or YV_ERR_UNSUPPORTED (and its message) for a pool of more bricks than
 // kMaxPoolBricks.
 yv_status pool_points_fit(uint32_t nbricks);
+// Whether a device pointer is on the boundary that a load or store of `bytes`
+// at a time needs (the kernels take pixels and packed lattice points whole).
+inline bool aligned_to(const void* p, uintptr_t bytes) {
+  return (reinterpret_cast<uintptr_t>(p) & (bytes - 1u)) == 0;
+}
+// The same for the arrays of a pool of the given precision.
+bool pool_aligned(const void* density, const void* albedo, int precision);
 
 // A host brick volume from parts built on the device (volume_host.cpp):
 // grids (ngrids x 64 refs), fp32 lattice values and RGB per brick, brick

@@ -400,6 +400,8 @@ def _make_function():
             ga = torch.empty(ashape, dtype=torch.float32, device=packed.device)
             desc = torch_desc(tv, packed=packed)
             grad_rgba = grad_rgba.contiguous()
+            if grad_rgba.data_ptr() % 16:  # a view that starts inside a pixel
+                grad_rgba = grad_rgba.clone()
             mp = L.MarchParams(float(alpha_scale), float(step_vox))
             L.check(L.lib.yv_volume_train_backward(
                 C.byref(desc), ca, len(ca), width, height, C.byref(mp),
