@@ -43,7 +43,7 @@ class DynamicSVO:
         if rgb is not None:
             try:
                 a = _pack_attr(rgb[0], rgb[1], rgb[2], 255, normal[0], normal[1], normal[2], 0)
-            except struct.error:  # not integers in range: as numpy takes or refuses them
+            except Exception:  # not integers in range: as numpy takes or refuses them
                 at = np.zeros(1, ATTR_DTYPE)
                 at["rgb"][0] = [rgb[0], rgb[1], rgb[2], 255]
                 at["n"][0] = [normal[0], normal[1], normal[2], 0]
