@@ -396,8 +396,14 @@ def _make_function():
         def backward(ctx, grad_rgba):
             packed, rgba = ctx.saved_tensors
             tv, ca, width, height, alpha_scale, step_vox, dshape, ashape = ctx.meta
-            gd = torch.empty(dshape, dtype=torch.float32, device=packed.device)
-            ga = torch.empty(ashape, dtype=torch.float32, device=packed.device)
+            points = packed.shape[0] * 729
+
+            def grad(shape, n):
+                # n values are written; an array that goes on past them has none there
+                make = torch.empty if shape.numel() == n else torch.zeros
+                return make(shape, dtype=torch.float32, device=packed.device)
+
+            gd, ga = grad(dshape, points), grad(ashape, 3 * points)
             desc = torch_desc(tv, packed=packed)
             grad_rgba = grad_rgba.contiguous()
             if grad_rgba.data_ptr() % 16:  # a view that starts inside a pixel
