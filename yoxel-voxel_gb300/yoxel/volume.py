@@ -245,6 +245,14 @@ def brick_bits(desc, stream=None):
     return out
 
 
+def _check_points(density, albedo, nb):
+    """The calls read nb * 729 fp32 densities and three times as many colours."""
+    for t, n in ((density, nb * 729), (albedo, 3 * nb * 729)):
+        if t.numel() * t.element_size() < 4 * n:
+            raise ValueError(f"{nb} bricks need {n} float32 values, got {tuple(t.shape)} "
+                             f"{t.dtype}")
+
+
 def pack_volume(density, albedo, out=None, stream=None):
     """(nbricks, 729, 4) float32 CUDA tensor of (r, g, b, density) per lattice
     point, from contiguous fp32 density (nbricks, 729) and albedo
@@ -253,6 +261,7 @@ def pack_volume(density, albedo, out=None, stream=None):
     nb = density.shape[0]
     if nb * 729 > 0xFFFFFFFF:  # (the call takes a 32-bit count)
         raise ValueError(f"{nb} bricks: more than 2^32 lattice points")
+    _check_points(density, albedo, nb)
     if out is None:
         out = torch.empty((nb, 729, 4), dtype=torch.float32, device=density.device)
     L.check(L.lib.yv_volume_pack(C.c_void_p(density.data_ptr()), C.c_void_p(albedo.data_ptr()),
@@ -377,6 +386,7 @@ def _make_function():
             density = density.contiguous()
             albedo = albedo.contiguous()
             nb = density.shape[0]
+            _check_points(density, albedo, nb)
             packed = torch.empty((nb, 729, 4), dtype=torch.float32, device=density.device)
             mask = torch.empty(nb * 17, dtype=torch.int32, device=density.device)
             desc = torch_desc(tv, packed=packed)
@@ -397,6 +407,9 @@ def _make_function():
             packed, rgba = ctx.saved_tensors
             tv, ca, width, height, alpha_scale, step_vox, dshape, ashape = ctx.meta
             points = packed.shape[0] * 729
+            for k in ("nbr_up", "nbr_dn"):
+                if tv[k].numel() < 7 * packed.shape[0]:
+                    raise ValueError(f"{k}: {tuple(tv[k].shape)} for {packed.shape[0]} bricks")
 
             def grad(shape, n):
                 # n values are written; an array that goes on past them has none there
