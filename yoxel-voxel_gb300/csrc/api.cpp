@@ -31,6 +31,7 @@ struct yv_renderer {
   // device scene
   uint2* d_nodes = nullptr;  // node records, 8 B each
   uint2* d_cold = nullptr;   // their cold records, 8 B each
+  uint32_t* d_child = nullptr;   // record of each node child, or null
   uint32_t* d_leaf_attr = nullptr;  // leaf -> attribute, or null
   uint4* d_attrs = nullptr;  // shading records, 16 B per attribute
   uint32_t* d_node_data = nullptr;  // level-of-detail attribute per node, or null
@@ -71,11 +72,13 @@ static yv_status cuda_fail(cudaError_t e, const char* what) {
 static void free_scene(yv_renderer* r) {
   cudaFree(r->d_nodes);
   cudaFree(r->d_cold);
+  cudaFree(r->d_child);
   cudaFree(r->d_leaf_attr);
   cudaFree(r->d_attrs);
   cudaFree(r->d_node_data);
   r->d_nodes = nullptr;
   r->d_cold = nullptr;
+  r->d_child = nullptr;
   r->d_leaf_attr = nullptr;
   r->d_attrs = nullptr;
   r->d_node_data = nullptr;
@@ -120,6 +123,8 @@ yv_status renderer_scene_buffers(yv_renderer* r, uint32_t nn, uint32_t na, uint2
   r->dyn = nullptr;
   cudaFree(r->d_node_data);
   r->d_node_data = nullptr;
+  cudaFree(r->d_child);
+  r->d_child = nullptr;
   cudaFree(r->d_leaf_attr);
   r->d_leaf_attr = nullptr;
   const size_t want_n = nn ? nn : 1, want_a = na ? na : 1;
@@ -246,7 +251,7 @@ static yv_status set_scene_impl(yv_renderer* r, const yv_vox_node* nodes, uint32
   YV_CUDA(cudaSetDevice(r->device), "cudaSetDevice");
   if (r->frame_pending) cudaStreamSynchronize(r->last_stream);
   free_scene(r);
-  const size_t nn = dl.records(), nl = dl.leaf_attr.size();
+  const size_t nn = dl.records(), nc = dl.child.size(), nl = dl.leaf_attr.size();
   if (nn) {
     YV_CUDA(cudaMalloc(&r->d_nodes, nn * 8u), "cudaMalloc(nodes)");
     YV_CUDA(cudaMalloc(&r->d_cold, nn * 8u), "cudaMalloc(ids)");
@@ -254,6 +259,11 @@ static yv_status set_scene_impl(yv_renderer* r, const yv_vox_node* nodes, uint32
             "upload nodes");
     YV_CUDA(cudaMemcpy(r->d_cold, dl.cold.data(), nn * 8u, cudaMemcpyHostToDevice),
             "upload ids");
+  }
+  if (nc) {
+    YV_CUDA(cudaMalloc(&r->d_child, nc * 4u), "cudaMalloc(children)");
+    YV_CUDA(cudaMemcpy(r->d_child, dl.child.data(), nc * 4u, cudaMemcpyHostToDevice),
+            "upload children");
   }
   if (nl) {
     YV_CUDA(cudaMalloc(&r->d_leaf_attr, nl * 4u), "cudaMalloc(leaves)");
@@ -288,12 +298,13 @@ static yv_status set_scene_impl(yv_renderer* r, const yv_vox_node* nodes, uint32
   r->cap_attrs = nattrs;
   r->scene.nodes = r->d_nodes;
   r->scene.cold = r->d_cold;
+  r->scene.child = r->d_child;
   r->scene.leaf_attr = r->d_leaf_attr;
   r->scene.attrs = r->d_attrs;
   r->scene.n_nodes = (uint32_t)nn;
   r->scene.n_attrs = nattrs;
   r->scene.root_word = dl.root_word;
-  r->scene_bytes = (uint64_t)nn * 16u + (uint64_t)nl * 4u + (uint64_t)nattrs * 16u;
+  r->scene_bytes = (uint64_t)nn * 16u + ((uint64_t)nc + nl) * 4u + (uint64_t)nattrs * 16u;
   r->scene_nodes = dl.n_unique;
   if (lod && nn) {
     YV_CUDA(cudaMalloc(&r->d_node_data, nn * 4u), "cudaMalloc(node data)");

@@ -111,8 +111,8 @@ __global__ void __launch_bounds__(256, kMinBlocks) batch_kernel(BatchLaunch b) {
 #pragma unroll 4
     for (int k = 0; k < kStepsPerVote; ++k)
       if ((mode == kPrimary || mode == kShadow) && r == kContinue)
-        r = trace_step<false, kBatchRing>(it.svo, nullptr, 0u, stk, ring, tr, mode == kShadow,
-                                          leaf, err);
+        r = trace_step<false, kBatchRing, false, false, true>(it.svo, nullptr, 0u, stk, ring, tr,
+                                                              mode == kShadow, leaf, err);
     if (r == kContinue) continue;
     if (mode == kShadow) {
       write_color(it.fa, off, r == kHit ? dark : lit, tr.fetches);

@@ -937,6 +937,7 @@ yv_status build_device_layout(const yv_vox_node* nodes, uint32_t count,
                               DeviceLayout* out, std::string* why) {
   out->nodes.clear();
   out->cold.clear();
+  out->child.clear();
   out->leaf_attr.clear();
   out->n_unique = 0;
   out->root_word = YV_DW_NULL;
@@ -949,6 +950,7 @@ yv_status build_device_layout(const yv_vox_node* nodes, uint32_t count,
   // iterative DFS: cycle check + height (levels of nodes)
   std::vector<uint8_t> color(count, 0);  // 0 new, 1 on stack, 2 done
   std::vector<uint8_t> height(count, 0);
+  uint64_t edges = 0;  // node children of the nodes reachable
   struct Frame { uint32_t id; int ch; };
   std::vector<Frame> st;
   st.push_back({root, 0});
@@ -990,6 +992,7 @@ yv_status build_device_layout(const yv_vox_node* nodes, uint32_t count,
       uint32_t w = n.child[ch];
       if (((n.flags >> ch) & 1u) || (w & 0x80000000u)) continue;
       hgt = std::max(hgt, 1 + (int)height[w]);
+      ++edges;
     }
     if (hgt > YV_MAX_DEPTH) {
       *why = "tree deeper than 16 node levels";
@@ -997,24 +1000,40 @@ yv_status build_device_layout(const yv_vox_node* nodes, uint32_t count,
     }
     height[fr.id] = (uint8_t)hgt;
     color[fr.id] = 2;
+    ++out->n_unique;
     st.pop_back();
   }
+  if (out->n_unique > YV_MAX_DEVICE_NODES) {
+    *why = "pool larger than 2^29 nodes";
+    return YV_ERR_BAD_POOL;
+  }
   out->depth = height[root];
-  // breadth-first records: the run of a node's children is laid down when its
-  // first record (first[id]) is reached, and shared by its other records.  The
-  // table of the leaves' attributes is kept from the first leaf on that is not
-  // numbered as its attribute.
+  // Breadth-first records, 16 bytes each with their cold half: one per parent
+  // edge, the run of a node's children laid down when its first record
+  // (first[id]) is reached and shared by its others - or, where that takes more
+  // memory than a table of 4 bytes per edge, one per node.  A pool with few
+  // shared nodes saves the load of the table entry; one that shares a lot would
+  // take up to 8 times its nodes (8 shared children a node: 128 bytes a node
+  // against 48).  The table of the leaves' attributes is kept from the
+  // first leaf on that is not numbered as its attribute.
+  const bool table = 16u * (edges + 1u) > 16u * (uint64_t)out->n_unique + 4u * edges ||
+                     edges >= YV_MAX_DEVICE_NODES;
   std::vector<uint32_t> first(count, 0xFFFFFFFFu);
   std::vector<uint32_t> order;  // record -> caller node id
-  order.reserve(count);
+  const size_t records = table ? (size_t)out->n_unique : (size_t)edges + 1u;
+  order.reserve(records);
   order.push_back(root);
-  out->nodes.reserve(2 * (size_t)count);
-  out->cold.reserve(2 * (size_t)count);
+  out->nodes.reserve(2 * records);
+  out->cold.reserve(2 * records);
+  if (table) {
+    out->child.reserve((size_t)edges);
+    first[root] = 0;
+  }
   uint64_t n_leaves = 0;
   bool same = true;
   for (size_t i = 0; i < order.size(); ++i) {
     const uint32_t id = order[i];
-    if (first[id] != 0xFFFFFFFFu) {
+    if (!table && first[id] != 0xFFFFFFFFu) {
       const size_t f = first[id];
       const uint32_t run = out->nodes[2 * f], codes = out->nodes[2 * f + 1],
                      leaf = out->cold[2 * f + 1];
@@ -1025,10 +1044,9 @@ yv_status build_device_layout(const yv_vox_node* nodes, uint32_t count,
       continue;
     }
     first[id] = (uint32_t)i;
-    ++out->n_unique;
     const yv_vox_node& n = nodes[id];
     uint32_t codes = 0, rank = 0;
-    out->nodes.push_back((uint32_t)order.size());
+    out->nodes.push_back((uint32_t)(table ? out->child.size() : order.size()));
     out->cold.push_back(id);
     out->cold.push_back((uint32_t)n_leaves);
     for (int ch = 0; ch < 8; ++ch) {
@@ -1045,15 +1063,15 @@ yv_status build_device_layout(const yv_vox_node* nodes, uint32_t count,
         ++n_leaves;
       } else if (!(w & 0x80000000u)) {
         k = rank++;
-        order.push_back(w);
+        if (!table || first[w] == 0xFFFFFFFFu) {
+          if (table) first[w] = (uint32_t)order.size();
+          order.push_back(w);
+        }
+        if (table) out->child.push_back(first[w]);
       }
       codes |= k << (28 - 4 * ch);
     }
     out->nodes.push_back(codes);
-    if (order.size() > YV_MAX_DEVICE_NODES || n_leaves > 0xFFFFFFFEull) {
-      *why = "pool larger than 2^29 nodes";
-      return YV_ERR_BAD_POOL;
-    }
   }
   out->root_word = 0;
   return YV_OK;

@@ -67,10 +67,11 @@ uint32_t frame_lanes(const SvoFrameArgs& a, uint64_t warps) {
   return lanes;
 }
 
-template <int kMinBlocks, bool kStaged, bool kLod = false, bool kRef = false>
+template <int kMinBlocks, bool kStaged, bool kLod = false, bool kRef = false,
+          bool kShared = false>
 static cudaError_t launch_with(const SvoDeviceScene& sc, const SvoFrameArgs& a, int bt,
                                uint32_t nsm, uint32_t refill, int per_sm, cudaStream_t stream) {
-  auto kern = svo_frame_kernel<kMinBlocks, kRef, kSvoRing, kStaged, kLod>;
+  auto kern = svo_frame_kernel<kMinBlocks, kRef, kSvoRing, kStaged, kLod, kShared>;
   const size_t smem = (size_t)(nsm / 2) * 16u + (size_t)(bt / 32) * kSvoRing * 1024u;
   if (smem > 48u * 1024u) {
     static bool opted_in[64] = {false};
@@ -130,6 +131,18 @@ cudaError_t launch_svo_frame(const SvoDeviceScene& sc, const SvoFrameArgs& a,
     // a caller VoxNode pool (an editable scene's device mirror): checked
     // traversal, the default launch shape
     e = launch_with<3, false, false, true>(sc, a, bt, 0, refill, 0, stream);
+  } else if (sc.child) {
+    // a pool that shares many of its nodes (one more load per descent): unstaged,
+    // at the two budgets that large and small frames run at by default.
+    // 1920x1080 / 320x240 of 377 nodes with 50 a level: 255 / 70 us; 244 / 68
+    // with a record per parent
+    const bool lod = a.lod_coef > 0.f && sc.node_data;
+    if (mb <= 4)
+      e = lod ? launch_with<3, false, true, false, true>(sc, a, bt, 0, refill, 0, stream)
+              : launch_with<3, false, false, false, true>(sc, a, bt, 0, refill, 0, stream);
+    else
+      e = lod ? launch_with<5, false, true, false, true>(sc, a, bt, 0, refill, 0, stream)
+              : launch_with<5, false, false, false, true>(sc, a, bt, 0, refill, 0, stream);
   } else if (a.lod_coef > 0.f && sc.node_data) {
     // level-of-detail frames: unstaged, the register budget as above (641x479
     // with a cut-off of 4: 94.0 us at 5, 89.1 at 4, 88.4 at 3)

@@ -17,7 +17,7 @@
 // 1D texture (reaction/report/main.tex:36-67).  On the device a traversal
 // reads one 8-byte record per node it enters, kept in registers while the
 // ray is in the node:
-//   .x  record of the first node child; the node children of a node are
+//   .x  record of the first node child; the records of the node children are
 //       consecutive in child order
 //   .y  a nibble per child, child c in bits 28 - 4 c and up :
 //       0..7 a node, record .x + this; 8 null; 12 a leaf
@@ -26,7 +26,9 @@
 // index to its attribute where the pool does not already number them so).
 // Records are breadth-first from the root, so the top levels come first.
 // A node that several parents share has one record per parent, all pointing
-// at the one run of its children.
+// at the one run of its children; in a pool that shares so much that this takes
+// more memory, a node has one record and `.x` is the place of its first node
+// child in a table of records, `child`.
 //
 // The traversal of a caller's VoxNode pool folds its flags into child words:
 //   word & YV_DW_LEAF  -> leaf, low 31 bits = VoxData (leaf attribute index)
@@ -59,6 +61,7 @@ namespace yv {
 struct DeviceLayout {
   std::vector<uint32_t> nodes;      // 2 per record: first node child, child codes
   std::vector<uint32_t> cold;       // 2 per record: caller node id, first leaf
+  std::vector<uint32_t> child;      // record of each node child; empty: consecutive
   std::vector<uint32_t> leaf_attr;  // attribute of each leaf; empty: its index
   uint32_t n_unique = 0;            // nodes reachable from the root
   uint32_t root_word = YV_DW_NULL;  // record of the root, or YV_DW_NULL

@@ -14,6 +14,7 @@ struct SvoDeviceScene {
   // 40-byte VoxNodes
   const void* nodes = nullptr;
   const uint2* cold = nullptr;          // {caller node id, first leaf} per record
+  const uint32_t* child = nullptr;      // record of each node child, or null: consecutive
   const uint32_t* leaf_attr = nullptr;  // leaf -> attribute, or null: the same index
   // library layout: 16-byte shading records {RGBA8, unit normal xyz fp32};
   // caller VoxNode pools: the caller's yv_leaf_attr (8 bytes)
