@@ -504,10 +504,9 @@ static yv_status run_backward(const yv_volume_device* vol, const yv_camera* cams
   const size_t npts = (size_t)vol->nbricks * 729u;
   float4* scratch = nullptr;
   a->ncams = ncams < kMaxVolumeCams ? ncams : kMaxVolumeCams;
-  // edge records while the pool keeps a scratch of their size between calls
-  // with room to spare (it holds on to 4 GiB), and where they can be had
+  // edge records where they pay and can be had
   size_t bytes = npts * sizeof(float4);
-  bool edges = bytes <= (1ull << 30) && backward_uses_edges(*a);
+  bool edges = backward_uses_edges(*a, (uint64_t)ncams * px);
   cudaError_t e = cudaSuccess;
   if (npts) {
     e = scratch_alloc(reinterpret_cast<void**>(&scratch), bytes * (edges ? 2u : 1u), s);

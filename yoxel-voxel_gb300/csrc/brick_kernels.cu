@@ -147,7 +147,7 @@ __device__ __forceinline__ float sample_dsigma(const VolumeArgs* a, float gc, fl
 // of 16 bytes for either.  64-camera fitting step of a 128^3 volume 8.46 -> 7.51
 // ms with edges; a launch that does not fill the GPU is bound by its longest
 // warp, not by atomics, and keeps the smaller scratch (4 cameras at 64x64: 494
-// us, 542 with edges).
+// us, 542 with edges), as do others where edges don't pay (backward_uses_edges).
 template <bool kEdges>
 struct GradVis {
   const VolumeArgs* a;
@@ -433,7 +433,20 @@ cudaError_t launch_volume_forward(VolumeArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-bool backward_uses_edges(VolumeArgs& a) {
+// Edge records (GradVis) pay where the launch is bound by its atomics and the
+// doubled scratch costs little.  Backward of smooth noise in trees of 128^3 and
+// 512^3 voxels, ms without / with them:
+//  * a scratch that leaves L2 (129 MB) turns the atomics it saves into DRAM
+//    traffic.  4 M rays: 3.9 k bricks (90 MB with edges) 9.81 / 7.99; 16.8 M
+//    rays: 4.9 k 8.18 / 8.09, 9.5 k (221 MB) 13.73 / 13.61, 14 k 19.4 / 19.4,
+//    26 k 31.0 / 31.5, 64 k bricks 50.4 / 51.8;
+//  * with few rays its zeroing and fold are not earned back.  3.9 k bricks, rays
+//    per lattice point 0.04: 0.99 / 1.10, 0.09: 1.32 / 1.31, 0.19: 2.04 / 1.86.
+// How many of the cells hold colour is known on the device only: where all do,
+// nothing is saved (4.1 k bricks, 4 M rays 10.6 / 10.9, half of them 10.5 / 9.8).
+bool backward_uses_edges(VolumeArgs& a, uint64_t rays) {
+  const uint64_t points = (uint64_t)a.v.nbricks * (uint64_t)kL3;
+  if (points * 32u > 128u << 20 || rays * 6u < points) return false;
   const uint32_t tiles = tile_ids(a);
   set_lanes(a, tiles);
   return !fits_small(march_blocks(a, tiles));

@@ -71,9 +71,9 @@ cudaError_t launch_volume_forward(VolumeArgs& a, cudaStream_t s);
 // Warp tiles of one camera's width x height frame in the march's order:
 // 16x16-pixel squares (row-major) of 8 tiles of 8x4 pixels.
 uint32_t volume_tiles_per_camera(int width, int height);
-// Whether a backward whose largest launch is a's keeps edge records (two float4
-// per lattice point) in its gradient scratch.
-bool backward_uses_edges(VolumeArgs& a);
+// Whether a backward of `rays` rays whose largest launch is a's keeps edge
+// records (two float4 per lattice point) in its gradient scratch.
+bool backward_uses_edges(VolumeArgs& a, uint64_t rays);
 cudaError_t launch_volume_backward(VolumeArgs& a, bool edges, cudaStream_t s);
 // packed[i] = (albedo rgb, density) of n lattice points (fp32 layouts).
 cudaError_t launch_pack_f32(const float* density, const float* albedo, uint32_t n,
