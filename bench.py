@@ -1340,9 +1340,8 @@ def run_ssna(args, cfg):
     post_ms = max(mean - mean_trace, 1e-6)
     # algorithmic bytes of the post chain per pixel: depth (albedo + t in, z
     # out: 12), each blur pass launched (z in + out: 8), shading (albedo, z,
-    # stored normal in, rgba out: 24); the limits of 2 passes reach the scene
-    # (the ncu launch list of the same command)
-    blurs = min(2, cfg["passes"])
+    # stored normal in, rgba out: 24)
+    blurs = r.ssna_passes(p)
     post_bytes = npix * (12 + 8 * blurs + 24)
     peaks, peak_kind = measured_peaks()
     achieved = post_bytes / (post_ms / 1e3) / 1e9
@@ -1377,7 +1376,8 @@ def run_ssna(args, cfg):
                 "path": "yv_render_ssna (C ABI) + frame copy into pinned host memory"},
         # trace, depth, blur passes and shading
         "gpu_launches": (int(st["launches"]) + 2 + blurs) * args.steps,
-        "gpu_launches_source": "ncu launch list, profiles/ssna_post_chain_1080p.md",
+        "gpu_launches_source": "trace launches of the frame's counters, depth, the blur passes "
+                               "that yv_ssna_passes counts, shading",
         "clocks": clocks})
     if not args.no_cpu_baseline:
         from oracle import ssna as O

@@ -715,6 +715,11 @@ yv_status yv_render_ssna(yv_renderer* r, const yv_ssna_params* p,
                          void* device_rgba, void* device_depth,
                          void* device_normals, void* stream);
 
+/* The blur passes of such a frame that are launched: of blur_passes, those
+ * whose limit is not below every depth that the unit cube has from the
+ * renderer's camera. */
+yv_status yv_ssna_passes(const yv_renderer* r, const yv_ssna_params* p, int32_t* passes);
+
 /* DumpTraceData into host arrays (each optional): dist = the hit's ray
  * distance (0 for a miss), color = the hit leaf's Color32 (0 for a miss),
  * normal = its unit normal (3 floats, 0 for a miss).  Synchronous. */

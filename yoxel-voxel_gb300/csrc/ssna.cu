@@ -467,6 +467,30 @@ double least_depth(const View& v) {
   return m * (1.0 - 1.0 / 128.0) - 1.0 / 1024.0;
 }
 
+// The blur passes to launch.  Pass i blurs z <= 5 voxSize / (pixelAng *
+// blurSize), blurSize = 3 (i + 1); pixel angle = fov / width in radians
+// (RenderParams::pixelAng).  A pass whose limit lies below every depth the scene
+// can have returns at once (pass_runs), as do those after it: they are not
+// launched.  Such a launch costs about 4 us of a frame: 1920x1080 from 1.5 scene
+// sides away needs 2 of the 5 default passes, 365 -> 353 us.
+PassLimits pass_limits(const yv_renderer_view& rv, const View& v, const yv_ssna_params& p) {
+  const double pix = (double)rv.fov_deg * (3.14159265358979323846 / 180.0) / v.width;
+  const double least = least_depth(v);
+  PassLimits pl;
+  pl.n = 0;
+  for (int i = 0; i < (p.ssna ? p.blur_passes : 0); ++i) {
+    pl.z[i] = (float)(5.0 * p.voxel_size / (pix * 3.0 * (i + 1)));
+    if (pl.z[i] < least) break;
+    pl.n = i + 1;
+  }
+  return pl;
+}
+
+bool params_ok(const yv_ssna_params* p) {
+  return p->blur_passes >= 0 && p->blur_passes <= kMaxPasses && p->voxel_size > 0.f &&
+         p->edge_threshold >= 0.f && p->edge_pad >= 0.f && !std::isnan(p->specular_exp);
+}
+
 yv_status ssna_fail(cudaError_t e, const char* what) {
   set_last_error(std::string("ssna: ") + what + ": " + cudaGetErrorString(e));
   cudaGetLastError();
@@ -515,12 +539,18 @@ yv_status yv_ssna_defaults(const yv_renderer* r, yv_ssna_params* p) {
   return YV_OK;
 }
 
+yv_status yv_ssna_passes(const yv_renderer* r, const yv_ssna_params* p, int32_t* passes) {
+  if (!r || !p || !passes || !params_ok(p)) return YV_ERR_INVALID_ARG;
+  yv_renderer_view rv;
+  if (!renderer_view(r, &rv)) return YV_ERR_NO_SCENE;
+  *passes = pass_limits(rv, make_view(rv), *p).n;
+  return YV_OK;
+}
+
 yv_status yv_render_ssna(yv_renderer* r, const yv_ssna_params* p, void* device_rgba,
                          void* device_depth, void* device_normals, void* stream) {
   if (!r || !p || !device_rgba) return YV_ERR_INVALID_ARG;
-  if (p->blur_passes < 0 || p->blur_passes > 64 || !(p->voxel_size > 0.f) ||
-      !(p->edge_threshold >= 0.f) || !(p->edge_pad >= 0.f) || std::isnan(p->specular_exp))
-    return YV_ERR_INVALID_ARG;
+  if (!params_ok(p)) return YV_ERR_INVALID_ARG;
   yv_renderer_view rv;
   if (!renderer_view(r, &rv)) return YV_ERR_NO_SCENE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -559,9 +589,6 @@ yv_status yv_render_ssna(yv_renderer* r, const yv_ssna_params* p, void* device_r
     std::memcpy(sh.latt[k], L.attenuation, 12);
   }
   const BlurWeights bw = blur_weights();
-  // pixel angle = fov / width in radians (RenderParams::pixelAng); pass i
-  // blurs z <= 5 voxSize / (pixelAng * blurSize), blurSize = 3 (i + 1)
-  const double pix = (double)rv.fov_deg * (3.14159265358979323846 / 180.0) / v.width;
   const float thr = p->edge_threshold;
   const float pad_thr = p->edge_pad * thr;
 
@@ -571,19 +598,10 @@ yv_status yv_render_ssna(yv_renderer* r, const yv_ssna_params* p, void* device_r
   depth_kernel<<<grd, blk, 0, s>>>(alb.as<uint32_t>(), ht.as<float>(), v, za.as<float>(),
                                    zmin.as<uint32_t>());
   if ((e = cudaGetLastError()) != cudaSuccess) return ssna_fail(e, "depth launch");
-  // A pass whose limit lies below every depth the scene can have returns at
-  // once (pass_runs), as do those after it: they are not launched.  Such a
-  // launch costs about 4 us of a frame: 1920x1080 from 1.5 scene sides away
-  // needs 2 of the 5 default passes, 365 -> 353 us.
-  const double least = least_depth(v);
-  PassLimits pl;
-  pl.n = 0;
+  const PassLimits pl = pass_limits(rv, v, *p);
   float* src = za.as<float>();
   float* dst = zb.as<float>();
-  for (int i = 0; i < passes; ++i) {
-    pl.z[i] = (float)(5.0 * p->voxel_size / (pix * 3.0 * (i + 1)));
-    if (pl.z[i] < least) break;
-    pl.n = i + 1;
+  for (int i = 0; i < pl.n; ++i) {
     blur_kernel<<<grd, blk, 0, s>>>(src, dst, v.width, v.height, pl.z[i], thr, pad_thr, bw,
                                     zmin.as<uint32_t>());
     if ((e = cudaGetLastError()) != cudaSuccess) return ssna_fail(e, "blur launch");

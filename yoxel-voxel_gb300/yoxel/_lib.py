@@ -233,6 +233,7 @@ _SIGS = {
                                   C.c_int32, C.c_int32, C.POINTER(FrameOutputs), P]),
     "yv_render_svo_noalloc_status": (S, [P, C.POINTER(U32)]),
     "yv_ssna_defaults": (S, [P, C.POINTER(SsnaParams)]),
+    "yv_ssna_passes": (S, [P, C.POINTER(SsnaParams), C.POINTER(C.c_int32)]),
     "yv_render_ssna": (S, [P, C.POINTER(SsnaParams), P, P, P, P]),
     "yv_renderer_trace_dump": (S, [P, P, P, P]),
 }

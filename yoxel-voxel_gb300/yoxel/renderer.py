@@ -269,6 +269,14 @@ class Renderer:
         lp.attenuation[:] = [float(v) for v in attenuation]
         lp.enabled = 1 if enabled else 0
 
+    def ssna_passes(self, params=None):
+        """Blur passes of an SSNA frame that are launched (a pass that reaches
+        no depth of the scene's cube is not)."""
+        n = C.c_int32()
+        L.check(L.lib.yv_ssna_passes(self._h, C.byref(params or self.ssna_params()), C.byref(n)),
+                "yv_ssna_passes")
+        return n.value
+
     def render_ssna(self, params=None, rgba=None, depth=None, normals=None, stream=None):
         """Enqueues an SSNA frame into CUDA tensors: rgba (h, w) int32
         (allocated when None), optional depth (h, w) float32 and normals
