@@ -73,7 +73,8 @@ static cudaError_t launch_with(const SvoDeviceScene& sc, const SvoFrameArgs& a, 
                                uint32_t nsm, uint32_t refill, int per_sm, cudaStream_t stream) {
   auto kern = svo_frame_kernel<kMinBlocks, kRef, kSvoRing, kStaged, kLod, kShared>;
   const size_t smem = (size_t)(nsm / 2) * 16u + (size_t)(bt / 32) * kSvoRing * 1024u;
-  if (smem > 48u * 1024u) {
+  // (48 KB without the opt-in, the kernel's few static words included)
+  if (smem > 40u * 1024u) {
     static bool opted_in[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
