@@ -361,6 +361,7 @@ const int32_t*  yv_volume_neighbors(const yv_volume_host* v, int upper);
 #define YV_PRECISION_F32_PACKED 2 /* float4 (r, g, b, density) (learnable) */
 #define YV_PRECISION_F16_PACKED 3 /* 8 B {fp16 density | r<<16 | g<<24, b},
                                      RGB8 (render only)                     */
+/* The densities of the two fp16 formats are finite (uploads saturate). */
 
 /* GPU build of the brick volume from a dense DEVICE lattice of (S+1)^3
  * floats, S = 8 * 4^levels, x fastest (index x + (S+1)*(y + (S+1)*z)), with

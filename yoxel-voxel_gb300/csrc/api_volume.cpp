@@ -35,9 +35,9 @@ yv_status fail(cudaError_t e, const char* what) {
   return e == cudaErrorMemoryAllocation ? YV_ERR_OUT_OF_MEMORY : YV_ERR_CUDA;
 }
 
-// IEEE binary32 -> binary16, round to nearest even, saturating at +-65504
-// (the fp16 lattice formats hold finite values only; the device decodes
-// them with exact bit arithmetic that assumes a finite half).  NaN -> 0.
+// IEEE binary32 -> binary16, round to nearest even, saturating at +-65504: the
+// fp16 lattice formats hold finite values only (the march multiplies a density by
+// weights that may be 0).  NaN -> 0.
 uint16_t f32_to_f16(float f) {
   uint32_t x;
   std::memcpy(&x, &f, 4);
@@ -310,7 +310,7 @@ yv_status yv_volume_upload(const yv_volume_host* v, int32_t precision, yv_volume
     abuf.resize(abytes);
     float* af = reinterpret_cast<float*>(abuf.data());
     for (size_t i = 0; i < n; ++i) {
-      for (int c = 0; c < 3; ++c) af[i * 4 + (size_t)c] = (float)alb[i * 3 + (size_t)c] * (1.0f / 255.0f);
+      for (size_t c = 0; c < 3; ++c) af[i * 4 + c] = (float)alb[i * 3 + c] * (1.0f / 255.0f);
       af[i * 4 + 3] = den[i];
     }
   } else {

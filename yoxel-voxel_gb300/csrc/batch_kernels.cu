@@ -79,8 +79,8 @@ __global__ void __launch_bounds__(256, kMinBlocks) batch_kernel(BatchLaunch b) {
         off = (uint32_t)y * (uint32_t)it.width + (uint32_t)x;
         if (it.kind == kBatchSvo) {
           pixel_dir(it.fa, x, y, dx, dy, dz);
-          if (begin_trace(it.svo, nullptr, 0u, it.fa.pos[0], it.fa.pos[1], it.fa.pos[2], dx, dy, dz, tr,
-                          err)) {
+          if (begin_trace(it.svo, nullptr, 0u, it.fa.pos[0], it.fa.pos[1], it.fa.pos[2], dx, dy,
+                          dz, tr, err)) {
             mode = kPrimary;
           } else {
             write_miss(it.fa, off, tr.fetches);

@@ -80,7 +80,8 @@ __device__ __forceinline__ bool mask_pays(const VolumeArgs& a) {
 // format) 876 -> 740 us from the cell found by one round-down add instead of
 // a conversion and clamps, the fraction clamped by the add's saturation, and
 // the half decoded by one conversion; 704 us with blocks of 128 threads.
-// kSkip: the pool carries a cell occupancy mask (a learnable pool does not).
+// kSkip: the pool carries a cell occupancy mask (library-owned pools, and a
+// learnable pool that the fitting step's forward packs).
 template <int P, int kBlocks, bool kSkip>
 __global__ void __launch_bounds__(kMarchThreads, 2 * kBlocks) volume_forward_kernel(VolumeArgs a) {
   // the launch's tiles (a range of them for a frame split across GPUs)
@@ -381,6 +382,14 @@ void launch_forward(const VolumeArgs& a, uint32_t blocks, cudaStream_t s) {
     launch_march<volume_forward_kernel<P, kMinBlocks, kSkip>>(a, blocks, s);
 }
 
+template <int P>
+void launch_forward(const VolumeArgs& a, bool skip, uint32_t blocks, cudaStream_t s) {
+  if (skip)
+    launch_forward<P, true>(a, blocks, s);
+  else
+    launch_forward<P, false>(a, blocks, s);
+}
+
 template <int P, bool kEdges>
 void launch_backward(const VolumeArgs& a, uint32_t blocks, cudaStream_t s) {
   if (fits_small(blocks))
@@ -424,10 +433,10 @@ cudaError_t launch_volume_forward(VolumeArgs& a, cudaStream_t s) {
   const uint32_t blocks = march_blocks(a, tiles);
   const bool skip = a.v.cell_mask != nullptr;
   switch (a.v.precision) {
-    case 0: skip ? launch_forward<0, true>(a, blocks, s) : launch_forward<0, false>(a, blocks, s); break;
-    case 1: skip ? launch_forward<1, true>(a, blocks, s) : launch_forward<1, false>(a, blocks, s); break;
-    case 2: skip ? launch_forward<2, true>(a, blocks, s) : launch_forward<2, false>(a, blocks, s); break;
-    case 3: skip ? launch_forward<3, true>(a, blocks, s) : launch_forward<3, false>(a, blocks, s); break;
+    case 0: launch_forward<0>(a, skip, blocks, s); break;
+    case 1: launch_forward<1>(a, skip, blocks, s); break;
+    case 2: launch_forward<2>(a, skip, blocks, s); break;
+    case 3: launch_forward<3>(a, skip, blocks, s); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -587,12 +596,11 @@ cudaError_t launch_pack_train(const float* density, const float* albedo, uint32_
   return cudaGetLastError();
 }
 
-// Unpack and apron fold in one pass over the lattice points (3072 bricks: 14
-// us, 27 from edge records, where an unpack, two gathers, two scatters and the zeroing of two
-// tensors took 105): a point's owner
-// (its own brick, or the upper neighbour for an apron point) sums its copies
-// in the order of fold_gather_kernel.  Interior points have one copy and need
-// no neighbour.
+// Unpack and apron fold in one pass over the lattice points: a point's owner
+// (its own brick, or the upper neighbour for an apron point) sums its copies in
+// the order of fold_gather_kernel.  Interior points have one copy and need no
+// neighbour.  3072 bricks: 14 us, 27 from edge records, where an unpack, two
+// gathers, two scatters and the zeroing of two tensors took 105.
 template <bool kEdges>
 __global__ void __launch_bounds__(256) fold_grads_kernel(const float4* __restrict__ p,
                                                          const int32_t* __restrict__ up,

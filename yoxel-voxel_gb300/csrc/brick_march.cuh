@@ -26,7 +26,8 @@
 //   d out_k / d c_jk    = T alpha_j            (c_A = 1)
 // Gradients for the 8 trilinear corners are coalesced in registers while
 // consecutive samples of a ray stay in the same trilinear cell, then flushed
-// with one 16-byte FP32 vector atomic per corner (brick_kernels.cu).
+// with FP32 vector atomics: one of 16 bytes per corner, or per edge of the cell
+// in x one of 8 bytes (no colour) or two of 16 (GradVis in brick_kernels.cu).
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -47,7 +48,6 @@ __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float ffma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ float lerpf_(float a, float b, float t) { return ffma(t, fsub(b, a), a); }
 
 // Exact conversions on the ALU / FMA pipes instead of the conversion unit
 // (which runs at a fraction of their rate); used where they measured faster

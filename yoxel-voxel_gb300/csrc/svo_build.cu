@@ -303,8 +303,8 @@ __host__ __device__ __forceinline__ uint32_t level_words(int k) {
   return k < 2 ? 1u : 1u << (3 * k - 6);
 }
 
-// Pass 3a: level k from level k+1; node and full are the arrays of all levels,
-// at[k] the first word of level k.
+// Pass 3a: the bytes `node` and `full` of level k from the words cn, cf of level
+// k+1 (a word holds the children of 8 regions).
 __global__ void fold_kernel(const uint64_t* cn, const uint64_t* cf, uint32_t words, uint8_t* node,
                             uint8_t* full) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -113,12 +113,13 @@ cudaError_t launch_svo_frame(const SvoDeviceScene& sc, const SvoFrameArgs& a,
   uint32_t refill = (uint32_t)(cfg.tile_rays <= 0 ? 32 : cfg.tile_rays);
   if (refill > 32) refill = 32;
   // register budget: blocks_per_sm 2 (up to 128 regs), 3 (80), 4 (64), 5
-  // (51).  0 = by the frame's size: 5 (fastest on the 2048^3 frame with
-  // unstaged node reads: 0.991 ms against 1.003 at 4 and 1.105 at 3; 6
-  // blocks spill), fewer while the frame holds under two 8x4-pixel tiles
-  // per resident warp, down to 3 (a warp takes a tile at a time, so a small
-  // frame ends on the warps that took two: the 512^2 frame 0.108 ms at 5,
-  // 0.104 at 4, 0.100 at 3)
+  // (51).  0 = by the frame's size: 5, fewer while the frame holds under two
+  // 8x4-pixel tiles per resident warp, down to 3 (such a frame ends with its
+  // slowest warps, and a warp is faster with more registers).  2048^3 terrain
+  // with shadow rays, us at 3 / 4 / 5 (L2 flushed): 3840x2160 (43 tiles per
+  // warp at 5) 2774 / 2798 / 2739, 1920x1080 853 / 859 / 850, 1280x720 471 /
+  // 472 / 471, 512x512 (1.4 tiles) 223 / 224 / 232, 320x240 195 / 195 / 205;
+  // 2 is slower from 1024x768 on (400 against 360); 6 spills
   int mb = cfg.blocks_per_sm > 5 ? 5 : cfg.blocks_per_sm;
   if (mb <= 0) {
     const uint64_t tiles = (a.id_end - a.id_begin) / 32u;

@@ -214,7 +214,7 @@ __global__ void mark_rows_flat_kernel(Lattice g, uint32_t* R) {
 // 4x4 square of (cy, cz): lane j and j + 16 OR the lower and upper rows of
 // square cell j, then the nibbles of the 16 lanes make the 64-cell mask (bit
 // x | y<<2 | z<<4) of each last-level node of the word.
-// counts[0] += nodes with a cell, counts[1] += cells.
+// node_count += nodes with a cell, cell_count += cells.
 __global__ void __launch_bounds__(256) mark_nodes_kernel(Lattice g, const uint32_t* R,
                                                          uint64_t* mask, uint32_t* node_count,
                                                          uint32_t* cell_count) {
@@ -727,8 +727,9 @@ yv_status upload_dense(const float* density, const uint8_t* rgb, int32_t levels,
   if (e == cudaSuccess && t.nbricks) {
     auto kern = precision == YV_PRECISION_F16          ? pack_bricks_kernel<YV_PRECISION_F16>
                 : precision == YV_PRECISION_F32        ? pack_bricks_kernel<YV_PRECISION_F32>
-                : precision == YV_PRECISION_F32_PACKED ? pack_bricks_kernel<YV_PRECISION_F32_PACKED>
-                                                       : pack_bricks_kernel<YV_PRECISION_F16_PACKED>;
+                : precision == YV_PRECISION_F32_PACKED
+                    ? pack_bricks_kernel<YV_PRECISION_F32_PACKED>
+                    : pack_bricks_kernel<YV_PRECISION_F16_PACKED>;
     kern<<<grid_for((uint64_t)t.nbricks * 32), 256, 0, s>>>(
         g, t.cells, t.nbricks, rgb_words(g), nullptr, nullptr, mem[1], mem[2], nullptr, t.map,
         static_cast<int32_t*>(mem[3]), static_cast<int32_t*>(mem[4]), mask, bits);
