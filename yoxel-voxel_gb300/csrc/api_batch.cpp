@@ -104,9 +104,13 @@ BatchLaunch launch_desc(const yv_batch* b) {
   // volumes share one (or that has none) runs the kernel carrying only that
   // march
   l.brick_precision = 3;
+  l.shared = false;
   bool first = true;
   for (const BatchItem& it : b->items) {
-    if (it.kind != kBatchBrick) continue;
+    if (it.kind != kBatchBrick) {
+      l.shared |= it.svo.child != nullptr;
+      continue;
+    }
     if (first) l.brick_precision = it.vol.precision;
     else if (l.brick_precision != it.vol.precision) l.brick_precision = -1;
     first = false;

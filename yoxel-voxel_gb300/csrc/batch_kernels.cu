@@ -32,7 +32,9 @@ __host__ __device__ __forceinline__ uint32_t item_table_vec4(int nitems) {
 
 // kP: the lattice format of every brick item (its march alone is compiled
 // in), or -1 for a batch mixing formats (all four marches).
-template <int kMinBlocks, int kP>
+// kShared: some SVO item has a table of children (the test of it at each descent
+// takes 1 % of a batch, so it is compiled out of the others).
+template <int kMinBlocks, int kP, bool kShared>
 __global__ void __launch_bounds__(256, kMinBlocks) batch_kernel(BatchLaunch b) {
   extern __shared__ uint4 dyn_smem[];
   BatchItem* items = reinterpret_cast<BatchItem*>(dyn_smem);
@@ -111,8 +113,8 @@ __global__ void __launch_bounds__(256, kMinBlocks) batch_kernel(BatchLaunch b) {
 #pragma unroll 4
     for (int k = 0; k < kStepsPerVote; ++k)
       if ((mode == kPrimary || mode == kShadow) && r == kContinue)
-        r = trace_step<false, kBatchRing, false, false, true>(it.svo, nullptr, 0u, stk, ring, tr,
-                                                              mode == kShadow, leaf, err);
+        r = trace_step<false, kBatchRing, false, false, kShared>(
+            it.svo, nullptr, 0u, stk, ring, tr, mode == kShadow, leaf, err);
     if (r == kContinue) continue;
     if (mode == kShadow) {
       write_color(it.fa, off, r == kHit ? dark : lit, tr.fetches);
@@ -148,9 +150,9 @@ __global__ void __launch_bounds__(256, kMinBlocks) batch_kernel(BatchLaunch b) {
   if (err) atomicOr(&b.counters[1], err);
 }
 
-template <int kMinBlocks, int kP>
+template <int kMinBlocks, int kP, bool kShared>
 cudaError_t launch_batch_with(const BatchLaunch& b, int bt, cudaStream_t s) {
-  auto kern = batch_kernel<kMinBlocks, kP>;
+  auto kern = batch_kernel<kMinBlocks, kP, kShared>;
   const size_t smem =
       (size_t)item_table_vec4(b.nitems) * 16u + (size_t)(bt / 32) * kBatchRing * 1024u;
   static bool opted_in[64] = {false};
@@ -176,11 +178,11 @@ cudaError_t launch_batch_with(const BatchLaunch& b, int bt, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-template <int kP>
+template <int kP, bool kShared = false>
 cudaError_t launch_by_budget(const BatchLaunch& b, int mb, int bt, cudaStream_t s) {
-  if (mb <= 2) return launch_batch_with<2, kP>(b, bt, s);
-  if (mb == 3) return launch_batch_with<3, kP>(b, bt, s);
-  return launch_batch_with<4, kP>(b, bt, s);
+  if (mb <= 2) return launch_batch_with<2, kP, kShared>(b, bt, s);
+  if (mb == 3) return launch_batch_with<3, kP, kShared>(b, bt, s);
+  return launch_batch_with<4, kP, kShared>(b, bt, s);
 }
 
 }  // namespace
@@ -196,6 +198,7 @@ cudaError_t launch_batch(const BatchLaunch& b, const LaunchCfg& cfg, cudaStream_
   int mb = cfg.blocks_per_sm > 4 ? 4 : cfg.blocks_per_sm;
   if (mb <= 0)
     mb = (uint64_t)b.total_ids / 32u >= 40ull * 16u * (uint64_t)device_sm_count() ? 3 : 2;
+  if (b.shared) return launch_by_budget<-1, true>(b, mb, bt, s);
   switch (b.brick_precision) {
     case 0: return launch_by_budget<0>(b, mb, bt, s);
     case 1: return launch_by_budget<1>(b, mb, bt, s);

@@ -36,6 +36,7 @@ struct BatchLaunch {
   uint32_t total_ids;
   uint32_t* counters;      // device scratch: [0] queue, [1] status
   int brick_precision;     // lattice format shared by every brick item, -1 if mixed
+  bool shared;             // some SVO item has a table of children
 };
 
 // Enqueues counter reset + the persistent batch kernel.
